@@ -14,7 +14,7 @@
 // the staged ranges (periodic images across a face, or ranges cut by the
 // shared-memory capacity) are read from global memory.
 //
-// The arithmetic and its order are those of contact_particle<PREC, 2>:
+// The arithmetic and its order are those of contact_warp<PREC, 2>:
 // topology visits the list in the reference's order with the reference's
 // slot policy; interact walks the occupied slots in slot order.  A slot that
 // topology did not hit in this step is released without evaluating it: its
@@ -395,7 +395,7 @@ __device__ __forceinline__ bool contact_particle_staged(const DevParams &P, cons
                            vb[q], wb[q], h, ra, rb, x_ab, len, delta_n);
                 S.delta_t_f[mempos] = h;
             } else {
-                V3 dt_new = contact_linear<PREC>(P, F, T3, es_dot, ev_dot, p, vel_a, angvel_a,
+                V3 dt_new = contact_linear<PREC>(P, F, T3, es_dot, ev_dot, ev_dot, p, vel_a, angvel_a,
                                                  vb[q], xyz(wb[q]), hd[q], ra, rb, x_ab, len,
                                                  delta_n);
                 S.delta_t[mempos] = make_double4(dt_new.x, dt_new.y, dt_new.z, 0.0);

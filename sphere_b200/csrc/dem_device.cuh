@@ -50,9 +50,12 @@ __device__ double contact_wall(const DevParams &P, V3 &F, V3 &T, double &es_dot,
 
 // contactLinear, src/contactmodels.cuh:241-408.  Returns the new
 // tangential displacement (zero where the reference leaves it unassigned).
+// The reference adds the normal and the tangential viscous dissipation one
+// after the other: ev_n and ev_t may be one accumulator, or two that the
+// caller adds in this order.
 template <int PREC>
 __device__ V3 contact_linear(const DevParams &P, V3 &F, V3 &T, double &es_dot,
-                             double &ev_dot, double &p, double4 vel_a, V3 angvel_a,
+                             double &ev_n, double &ev_t, double &p, double4 vel_a, V3 angvel_a,
                              double4 vel_b, V3 angvel_b, double4 dt0, double ra,
                              double rb, V3 x, double x_length, double delta)
 {
@@ -74,7 +77,7 @@ __device__ V3 contact_linear(const DevParams &P, V3 &F, V3 &T, double &es_dot,
     }
     V3 f_n = smul3(fmax(0.0, -k_n * delta + P.gamma_n * vel_n), n);
     double f_n_length = vlen<PREC>(f_n);
-    ev_dot += 0.5 * P.gamma_n * vel_n * vel_n;
+    ev_n += 0.5 * P.gamma_n * vel_n * vel_n;
     V3 f_c = smul3(-P.kappa * ssqrt<PREC>(ra * rb), n);
     V3 f_t = mk3(0.0, 0.0, 0.0);
     if (delta_t0_length > 0.0 || vel_t_length > 0.0) {
@@ -84,7 +87,7 @@ __device__ V3 contact_linear(const DevParams &P, V3 &F, V3 &T, double &es_dot,
         f_t = add3(f_t_elast, f_t_visc);
         double f_t_length = vlen<PREC>(f_t);
         double f_t_limit = P.mu_s * vlen<PREC>(sub3(f_n, f_c));
-        ev_dot += 0.5 * P.gamma_t * vel_t_length * vel_t_length;
+        ev_t += 0.5 * P.gamma_t * vel_t_length * vel_t_length;
         if (f_t_length > f_t_limit) {
             V3 t = divs3(f_t, vlen<PREC>(f_t));
             f_t = smul3(f_t_limit, t);
@@ -440,154 +443,401 @@ __device__ __forceinline__ void contact_walls(const DevParams &P, const DevState
     out.wf0 = wf0; out.wf1 = wf1; out.wf2 = wf2; out.wf3 = wf3; out.wf4 = wf4;
 }
 
-// Contact search + forces of sorted particle k (topology and interact of
-// the reference, walls included).  srow is the thread's slot scratch in
-// shared memory (entry i at srow[i * B + t]: the partner's original index).
-// Returns false after raising a capacity error.
+// Scratch of one warp of contact_warp in shared memory: the contacts of one
+// round, their results, and (model 2) the list entry that holds each slot.
+struct WarpScratch {
+    uint16_t *item;       // item[lane]: particle | slot or list entry << 5
+    double *d;            // result component c of lane l at d[c * 32 + l]
+    float *f;             // mixed: force and torque, which the law gives in FP32
+    uint8_t *entry;       // entry[particle * nc + slot], kNoEntry without one
+};
+constexpr unsigned kNoEntry = 0xffu;
+
+// Bytes of a warp's scratch: at most 10 result doubles per lane (mixed: 3
+// doubles and 6 floats), 32 items, 32 slot rows of nc (a multiple of 4 in
+// memory) entries.
+template <int PREC, int MODEL>
+__host__ __device__ constexpr size_t contact_warp_bytes(unsigned nc)
+{
+    return (PREC == 2 && MODEL == 2 ? 3 * 32 * 8 + 6 * 32 * 4 : 10 * 32 * 8) + 64 +
+           (MODEL == 2 ? 32 * (size_t)((nc + 3u) & ~3u) : 0);
+}
+
+template <int PREC, int MODEL>
+__device__ __forceinline__ WarpScratch contact_warp_scratch(unsigned char *block_base, unsigned warp,
+                                                            unsigned nc)
+{
+    unsigned char *base = block_base + warp * contact_warp_bytes<PREC, MODEL>(nc);
+    constexpr size_t res = contact_warp_bytes<PREC, 1>(0) - (PREC == 2 && MODEL == 2 ? 1024 : 0) - 64;
+    WarpScratch w;
+    w.d = reinterpret_cast<double *>(base);
+    w.f = reinterpret_cast<float *>(base + 3 * 32 * 8);
+    w.item = reinterpret_cast<uint16_t *>(base + res);
+    w.entry = base + res + 64;
+    return w;
+}
+
+// Particles per warp for np particles on `warps` resident warps: the fewest
+// that still give every particle a place in one wave, so small systems spread
+// their contacts over more lanes and large ones keep one particle per lane.
+// Measured (launch time of k_contacts): 20,000 spheres 27 us with one wave of
+// 8 per warp, 31 with two waves of 4 and 34 with half a wave of 16; 400
+// spheres 14 us with 2 per warp and 18 with 4.
+__host__ __device__ inline unsigned contact_pw(unsigned np, unsigned warps)
+{
+    unsigned pw = 32;
+    while (pw > 1 && (np + pw / 2 - 1) / (pw / 2) <= warps) pw /= 2;
+    return pw;
+}
+
+__device__ __forceinline__ unsigned warp_inclusive_sum(unsigned v)
+{
+    const unsigned lane = threadIdx.x & 31u;
+    for (unsigned d = 1; d < 32u; d <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += y;
+    }
+    return v;
+}
+
+// Whether list entry e of particle xa overlaps it: the reference's test
+// |x_ab| - (r_a + r_b) < 0 in the precision of the step.  The squared distance
+// settles it except within a band around the squared radius sum that covers
+// the rounding of the length (FP32: 6e-8 in the square, 6e-8 in the root;
+// FP64: 1e-15), where the length itself is compared.
+template <int TP>
+__device__ __forceinline__ bool touches(const DevParams &P, const double4 &xa, const double4 &xb,
+                                        uint32_t code)
+{
+    constexpr double band = TP == 0 ? 4e-7 : 1e-12;
+    V3 xab = mk3(xa.x - xb.x, xa.y - xb.y, xa.z - xb.z);
+    if (code) xab = add3(xab, dm_decode(P, (uint8_t)code));
+    const double d2 = dot3(xab, xab), rs = xa.w + xb.w, r2 = rs * rs;
+    if (d2 > r2 * (1.0 + band) && d2 > 1e-30) return false;
+    if (d2 < r2 * (1.0 - band) && d2 > 1e-30) return true;
+    return vlen<TP>(xab) - rs < 0.0;
+}
+
+// Contact search + forces of the sorted particles k0 .. k0 + pw - 1 (topology
+// and interact of the reference, walls included) by one warp; pw is a power
+// of two up to 32 and lane l < pw owns particle k0 + l, whose results `out`
+// receives.  Returns true in the lanes whose particle was evaluated (false
+// beyond np and after raising a capacity error).  All lanes must call it.
+//
+// The work of a particle is a long dependent chain (a dozen list candidates,
+// then a contact law of several hundred FP64 instructions per contact), and
+// its length differs between neighbouring particles.  So the warp shares it:
+//   1. list entries are tested by all lanes (32 / pw lanes per particle),
+//      four at a time so that their loads overlap;
+//      A partner that still holds the slot it held before (nl_slot, a hint
+//      that is checked against the row) has its slot at once;
+//   2. the owner runs the reference's slot policy (the first slot that holds
+//      the partner, else the last empty one) on the others, in list order.
+//      An entry that finds its slot changes none, so its turn is free;
+//   3. the occupied slots of the warp's particles, in (particle, slot) order,
+//      are evaluated 32 at a time, one per lane, whatever particle they
+//      belong to; results go to shared memory.  The list entry gives the
+//      partner's sorted position; a slot without one (its partner no longer
+//      overlaps, or lies outside the cells the search visits) takes it from
+//      the row;
+//   4. the owner adds its contacts' results in slot order, the reference's
+//      summation order, so every sum is formed as before, bit for bit.
+// Measured on the shear box (100,000 particles, B200, launch time): one
+// particle per thread 43 us mixed and 58 us faithful FP64; this 36 and 45 (400 spheres, 8 contacts each: 49 and
+// 14 us, and 54 and 18 us for the whole step).
 // PREC 0: faithful FP64, 1: FP64, 2: mixed (FP64 overlap, FP32 contact law,
 // FP64 accumulation).
 template <int PREC, int MODEL>
-__device__ __forceinline__ bool contact_particle(const DevParams &P, const DevState &S, unsigned k,
-                                                 uint32_t *srow, unsigned B, unsigned t,
-                                                 ContactOut &out)
+__device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState &S, unsigned k0,
+                                             unsigned pw, const WarpScratch &W, ContactOut &out)
 {
     constexpr int TP = PREC == 2 ? 1 : PREC;  // precision of overlap tests
-    const unsigned NC = P.nc;
-    const uint64_t full = NC >= 64 ? ~0ull : ((1ull << NC) - 1ull);
-    const unsigned o = S.orig_of[k];
-    const double4 xa = S.x[k];
-    const double ra = xa.w;
-    const double4 vel_a = S.vel[k];
-    const V3 angvel_a = xyz(S.angvel[k]);
-    double es_dot = 0.0, ev_dot = 0.0, p = 0.0;
-    V3 F = mk3(0.0, 0.0, 0.0), T = mk3(0.0, 0.0, 0.0);
-    const unsigned cnt = S.nl_count[k];
-    const size_t np = P.np;
+    constexpr unsigned ALL = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned ip = lane & (pw - 1u), sub = lane / pw, S_ = 32u / pw;
+    const unsigned np = P.np, NC = P.nc;
+    const unsigned k = k0 + ip;
+    const bool valid = k < np;
+    const bool owner = valid && sub == 0;
+    const double4 xa = valid ? S.x[k] : make_double4(0.0, 0.0, 0.0, 0.0);
+    const unsigned cnt = valid ? S.nl_count[k] : 0u;
+    // the capillary law reaches beyond contact, so it scans the cells
+    const bool scan = cnt == NL_OVERFLOW || (MODEL == 1 && P.db > 0.0 && P.kappa != 0.0);
 
+    uint64_t mask = 0;
+    size_t rowbase = 0;
+    unsigned o = 0;
+    if (MODEL == 2 && valid) {
+        o = S.orig_of[k];
+        rowbase = (size_t)o * NC;
+        mask = S.occ[o];
+    }
+
+    // ---- 1. overlapping list entries (at most nlmax <= 64) ----
+    // hits: model 1 all of them, model 2 those whose partner holds no slot yet
+    uint64_t hits = 0;
+    unsigned nhit = 0;
+    const unsigned ncp = (NC + 3u) & ~3u;   // row stride of W.entry
     if (MODEL == 2) {
-        const size_t rowbase = (size_t)o * NC;
-        uint64_t mask = S.occ[o];
-        uint64_t written = 0;
-        {
-            uint64_t m = mask;
-            while (m) {
-                int i = __ffsll((long long)m) - 1;
-                srow[i * B + t] = S.contacts[rowbase + i];
-                m &= m - 1;
+        for (unsigned i = lane; i < pw * ncp / 4u; i += 32u) reinterpret_cast<uint32_t *>(W.entry)[i] = 0xffffffffu;
+        __syncwarp();
+    }
+    {
+        const unsigned n = scan ? 0u : cnt;
+        uint64_t found = 0;
+        for (unsigned j0 = sub; j0 < n; j0 += 4u * S_) {
+            uint32_t e[4];
+            double4 xb[4];
+            bool touch[4];
+#pragma unroll
+            for (unsigned q = 0; q < 4; ++q) e[q] = j0 + q * S_ < n ? S.nl[(size_t)(j0 + q * S_) * np + k] : 0u;
+#pragma unroll
+            for (unsigned q = 0; q < 4; ++q)
+                if (j0 + q * S_ < n) xb[q] = S.x[e[q] & 0x0fffffffu];
+#pragma unroll
+            for (unsigned q = 0; q < 4; ++q) {
+                touch[q] = j0 + q * S_ < n && touches<TP>(P, xa, xb[q], e[q] >> 28);
+                if (MODEL == 1 && touch[q]) hits |= 1ull << (j0 + q * S_);
+            }
+            if (MODEL == 2) {
+                unsigned slot[4], bo[4];
+#pragma unroll
+                for (unsigned q = 0; q < 4; ++q)
+                    if (touch[q]) {
+                        slot[q] = S.nl_slot[(size_t)(j0 + q * S_) * np + k];
+                        bo[q] = S.orig_of[e[q] & 0x0fffffffu];
+                    }
+#pragma unroll
+                for (unsigned q = 0; q < 4; ++q)
+                    if (touch[q]) {
+                        const unsigned j = j0 + q * S_;
+                        ++nhit;
+                        if (slot[q] < NC && ((mask >> slot[q]) & 1ull) && S.contacts[rowbase + slot[q]] == bo[q]) {
+                            W.entry[ip * ncp + slot[q]] = (uint8_t)j;
+                            found |= 1ull << j;
+                        } else {
+                            hits |= 1ull << j;
+                        }
+                    }
             }
         }
-        // --- topology ---
-        int nc = 0;
-        bool ok = true;
-        auto visit = [&](unsigned b, int sx, int sy) -> bool {
-            double4 xb = S.x[b];
-            double rb = xb.w;
-            V3 xab = mk3(xa.x - xb.x, xa.y - xb.y, xa.z - xb.z);
-            xab = add3(xab, shift_vec(P, sx, sy));
-            double len = vlen<TP>(xab);
-            double delta = len - (ra + rb);
-            if (delta < 0.0) {
-                unsigned b_orig = S.orig_of[b];
-                int cpos = pick_slot(mask, full, srow, B, t, b_orig, nc);
-                if (cpos >= (int)NC || nc + 1 > (int)NC) {
-                    raise_err(S.ctl, DERR_CAPACITY, (int)o);
-                    ok = false;
-                    return false;
+        for (unsigned d = pw; d < 32u; d <<= 1) {
+            hits |= __shfl_xor_sync(ALL, hits, d);
+            if (MODEL == 2) nhit += __shfl_xor_sync(ALL, nhit, d);
+        }
+        if (MODEL == 2 && pw < 32u) {
+            // where two images of one partner touch, the later entry counts;
+            // different lanes may have seen them
+            __syncwarp();
+            while (__any_sync(ALL, found != 0)) {
+                if (found) {
+                    const unsigned j = (unsigned)__ffsll((long long)found) - 1u;
+                    const unsigned at = ip * ncp + S.nl_slot[(size_t)j * np + k];
+                    if (W.entry[at] < j) W.entry[at] = (uint8_t)j;   // seen again below
+                    else found &= found - 1;
                 }
-                srow[cpos * B + t] = b_orig;
-                mask |= 1ull << cpos;
-                written |= 1ull << cpos;
-                S.dmcode[rowbase + cpos] = dm_encode(sx, sy);
-                ++nc;
+                __syncwarp();
             }
-            return true;
-        };
-        if (cnt != NL_OVERFLOW) {
-            for (unsigned j = 0; j < cnt; ++j) {
-                uint32_t e = S.nl[(size_t)j * np + k];
-                uint32_t c = e >> 28;
-                int sx = (c & 1) ? 1 : ((c & 2) ? -1 : 0);
-                int sy = (c & 4) ? 1 : ((c & 8) ? -1 : 0);
-                if (!visit(e & 0x0fffffffu, sx, sy)) break;
-            }
-        } else {
-            for_each_cell_candidate(P, S, k, xa, visit);
         }
-        if (!ok) return false;
-        // --- interact, history contacts in slot order ---
-        uint64_t m = mask;
-        while (m) {
-            const int i = __ffsll((long long)m) - 1;
-            m &= m - 1;
-            const unsigned b_orig = srow[i * B + t];
-            if (b_orig >= P.np) { raise_err(S.ctl, DERR_CAPACITY, (int)o); return false; }
-            const size_t mempos = rowbase + i;
-            V3 dm = dm_decode(P, S.dmcode[mempos]);
-            unsigned kb = S.pos_of[b_orig];
-            double4 xb = S.x[kb];
-            double rb = xb.w;
-            V3 x_ab = mk3(xa.x - xb.x + dm.x, xa.y - xb.y + dm.y, xa.z - xb.z + dm.z);
-            double len = vlen<TP>(x_ab);
-            double delta_n = len - (ra + rb);
-            if (delta_n < 0.0) {
-                if constexpr (PREC == 2) {
-                    float4 h = S.delta_t_f[mempos];
-                    mixed_pair(P, F, T, es_dot, ev_dot, p, S.vel_f[k], S.angvel_f[k], S.vel_f[kb],
-                               S.angvel_f[kb], h, ra, rb, x_ab, len, delta_n);
-                    S.delta_t_f[mempos] = h;
-                } else {
-                    V3 dt_new = contact_linear<PREC>(P, F, T, es_dot, ev_dot, p, vel_a, angvel_a,
-                                                     S.vel[kb], xyz(S.angvel[kb]),
-                                                     S.delta_t[mempos], ra, rb, x_ab, len, delta_n);
-                    S.delta_t[mempos] = make_double4(dt_new.x, dt_new.y, dt_new.z, 0.0);
+    }
+
+    // ---- 2. slots of new contacts (model 2) ----
+    bool ok = owner;
+    const uint64_t mask0 = mask;
+    if (MODEL == 2) {
+        if (owner && (hits || scan || nhit > NC)) {
+            const uint64_t full = NC >= 64 ? ~0ull : ((1ull << NC) - 1ull);
+            // the slot of partner b_orig, or NC when the row is full
+            auto take = [&](unsigned b_orig, uint32_t code) -> unsigned {
+                unsigned slot = NC;
+                for (uint64_t m = mask; m; m &= m - 1) {
+                    const unsigned i = (unsigned)__ffsll((long long)m) - 1u;
+                    if (S.contacts[rowbase + i] == b_orig) { slot = i; break; }
+                }
+                if (slot == NC) {
+                    const uint64_t empty = ~mask & full;
+                    if (empty) slot = 63u - (unsigned)__clzll((long long)empty);
+                    else ok = false;
+                }
+                if (slot < NC) {
+                    S.contacts[rowbase + slot] = b_orig;
+                    S.dmcode[rowbase + slot] = (uint8_t)code;
+                    mask |= 1ull << slot;
+                }
+                return slot;
+            };
+            if (!scan) {
+                for (uint64_t m = hits; m && ok; m &= m - 1) {
+                    const unsigned j = (unsigned)__ffsll((long long)m) - 1u;
+                    const size_t at = (size_t)j * np + k;
+                    const uint32_t e = S.nl[at];
+                    const unsigned slot = take(S.orig_of[e & 0x0fffffffu], e >> 28);
+                    S.nl_slot[at] = (uint8_t)slot;
+                    if (slot < NC) {
+                        uint8_t &at_slot = W.entry[ip * ncp + slot];
+                        if (at_slot == kNoEntry || at_slot < j) at_slot = (uint8_t)j;
+                    }
                 }
             } else {
+                for_each_cell_candidate(P, S, k, xa, [&](unsigned b, int sx, int sy) -> bool {
+                    const uint32_t code = dm_encode(sx, sy);
+                    if (touches<TP>(P, xa, S.x[b], code)) {
+                        ++nhit;
+                        (void)take(S.orig_of[b], code);
+                    }
+                    return ok;
+                });
+            }
+            if (nhit > NC) ok = false;
+            if (!ok) {
+                // the row keeps the contacts it had
+                raise_err(S.ctl, DERR_CAPACITY, (int)o);
+                for (uint64_t m = mask & ~mask0; m; m &= m - 1)
+                    S.contacts[rowbase + (__ffsll((long long)m) - 1)] = np;
+            }
+        }
+    }
+
+    // ---- 3, 4. contacts, 32 at a time ----
+    double es_dot = 0.0, ev_dot = 0.0, p = 0.0;
+    V3 F = mk3(0.0, 0.0, 0.0), T = mk3(0.0, 0.0, 0.0);
+    uint64_t todo = ok ? (MODEL == 2 ? mask : hits) : 0ull;
+    const unsigned mine = __popcll(todo);
+    const unsigned end = warp_inclusive_sum(mine), beg = end - mine;
+    const unsigned total = __shfl_sync(ALL, end, 31);
+    __syncwarp();   // the rows and their entries
+    for (unsigned r0 = 0; r0 < total; r0 += 32u) {
+        for (unsigned q = max(beg, r0); q < min(end, r0 + 32u); ++q) {
+            W.item[q - r0] = (uint16_t)(ip | (unsigned)(__ffsll((long long)todo) - 1) << 5);
+            todo &= todo - 1;
+        }
+        __syncwarp();
+        bool released = false;
+        if (r0 + lane < total) {
+            const unsigned it = W.item[lane], ia = it & 31u, i = it >> 5, ka = k0 + ia;
+            const double4 xi = S.x[ka];
+            const double ra = xi.w;
+            V3 f = mk3(0.0, 0.0, 0.0), t = mk3(0.0, 0.0, 0.0);
+            double es = 0.0, ev_n = 0.0, ev_t = 0.0, pp = 0.0;
+            if (MODEL == 2) {
+                const size_t mempos = (size_t)S.orig_of[ka] * NC + i;
+                const unsigned j = W.entry[ia * ncp + i];
+                uint32_t e;   // the partner as a list entry has it
+                bool there = true;
+                if (j != kNoEntry) {
+                    e = S.nl[(size_t)j * np + ka];
+                    S.dmcode[mempos] = (uint8_t)(e >> 28);
+                } else {
+                    const unsigned b_orig = S.contacts[mempos];
+                    there = b_orig < np;
+                    e = there ? S.pos_of[b_orig] | (uint32_t)S.dmcode[mempos] << 28 : 0u;
+                }
+                if (!there) {
+                    raise_err(S.ctl, DERR_CAPACITY, (int)S.orig_of[ka]);
+                } else {
+                    const V3 dm = dm_decode(P, (uint8_t)(e >> 28));
+                    const unsigned kb = e & 0x0fffffffu;
+                    const double4 xb = S.x[kb];
+                    const double rb = xb.w;
+                    const V3 x_ab = mk3(xi.x - xb.x + dm.x, xi.y - xb.y + dm.y, xi.z - xb.z + dm.z);
+                    const double len = vlen<TP>(x_ab);
+                    const double delta_n = len - (ra + rb);
+                    if (delta_n < 0.0) {
+                        if constexpr (PREC == 2) {
+                            float4 h = S.delta_t_f[mempos];
+                            mixed_pair(P, f, t, es, ev_n, pp, S.vel_f[ka], S.angvel_f[ka],
+                                       S.vel_f[kb], S.angvel_f[kb], h, ra, rb, x_ab, len, delta_n);
+                            S.delta_t_f[mempos] = h;
+                        } else {
+                            const V3 dt_new = contact_linear<PREC>(
+                                P, f, t, es, ev_n, ev_t, pp, S.vel[ka], xyz(S.angvel[ka]), S.vel[kb],
+                                xyz(S.angvel[kb]), S.delta_t[mempos], ra, rb, x_ab, len, delta_n);
+                            S.delta_t[mempos] = make_double4(dt_new.x, dt_new.y, dt_new.z, 0.0);
+                        }
+                    } else {
+                        released = true;
+                        if constexpr (PREC == 2) S.delta_t_f[mempos] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        else S.delta_t[mempos] = make_double4(0.0, 0.0, 0.0, 0.0);
+                    }
+                }
+            } else {
+                // findAndProcessContactsInCell, contactsearch.cuh:91-186
+                const uint32_t e = S.nl[(size_t)i * np + ka];
+                const unsigned kb = e & 0x0fffffffu;
+                const double4 xb = S.x[kb];
+                V3 x_ab = mk3(xi.x - xb.x, xi.y - xb.y, xi.z - xb.z);
+                x_ab = add3(x_ab, dm_decode(P, (uint8_t)(e >> 28)));
+                const double len = vlen<TP>(x_ab);
+                contact_linear_viscous<TP>(P, f, t, pp, S.vel[ka], xyz(S.angvel[ka]), S.vel[kb],
+                                           xyz(S.angvel[kb]), ra, xb.w, x_ab, len, len - (ra + xb.w),
+                                           P.kappa);
+            }
+            double *d = W.d + lane;
+            if constexpr (PREC == 2 && MODEL == 2) {
+                float *g = W.f + lane;
+                g[0] = (float)f.x; g[32] = (float)f.y; g[64] = (float)f.z;
+                g[96] = (float)t.x; g[128] = (float)t.y; g[160] = (float)t.z;
+                d[0] = es; d[32] = ev_n; d[64] = pp;
+            } else {
+                d[0] = f.x; d[32] = f.y; d[64] = f.z;
+                d[96] = t.x; d[128] = t.y; d[160] = t.z;
+                d[192] = pp;
+                if (MODEL == 2) { d[224] = es; d[256] = ev_n; d[288] = ev_t; }
+            }
+        }
+        const unsigned rel = __ballot_sync(ALL, released);
+        __syncwarp();
+        for (unsigned q = max(beg, r0); q < min(end, r0 + 32u); ++q) {
+            const unsigned l = q - r0;
+            if ((rel >> l) & 1u) {
+                const unsigned i = W.item[l] >> 5;
                 mask &= ~(1ull << i);
-                written |= 1ull << i;
-                if constexpr (PREC == 2) S.delta_t_f[mempos] = make_float4(0.f, 0.f, 0.f, 0.f);
-                else S.delta_t[mempos] = make_double4(0.0, 0.0, 0.0, 0.0);
+                S.contacts[rowbase + i] = np;
+                continue;
+            }
+            const double *d = W.d + l;
+            if constexpr (PREC == 2 && MODEL == 2) {
+                const float *g = W.f + l;
+                F = add3(F, mk3(g[0], g[32], g[64]));
+                T = add3(T, mk3(g[96], g[128], g[160]));
+                es_dot += d[0];
+                ev_dot += d[32];
+                p += d[64];
+            } else {
+                F = add3(F, mk3(d[0], d[32], d[64]));
+                T = add3(T, mk3(d[96], d[128], d[160]));
+                p += d[192];
+                if (MODEL == 2) {
+                    es_dot += d[224];
+                    ev_dot += d[256];
+                    ev_dot += d[288];
+                }
             }
         }
-        if (written) {
-            uint64_t w = written;
-            while (w) {
-                int i = __ffsll((long long)w) - 1;
-                w &= w - 1;
-                S.contacts[rowbase + i] = (mask >> i) & 1ull ? srow[i * B + t] : P.np;
-            }
-            S.occ[o] = mask;
-        }
-    } else if (MODEL == 1) {
-        // findAndProcessContactsInCell, contactsearch.cuh:91-186
-        auto visit = [&](unsigned b, int sx, int sy) -> bool {
+        __syncwarp();
+    }
+    if (!ok) return false;
+    const double4 vel_a = S.vel[k];
+    const V3 angvel_a = xyz(S.angvel[k]);
+    if (MODEL == 2) {
+        if (mask != mask0) S.occ[o] = mask;
+    } else if (scan) {
+        for_each_cell_candidate(P, S, k, xa, [&](unsigned b, int sx, int sy) -> bool {
             double4 xb = S.x[b];
             double rb = xb.w;
             V3 x_ab = mk3(xa.x - xb.x, xa.y - xb.y, xa.z - xb.z);
             x_ab = add3(x_ab, shift_vec(P, sx, sy));
             double len = vlen<TP>(x_ab);
-            double delta_ab = len - (ra + rb);
+            double delta_ab = len - (xa.w + rb);
             if (delta_ab < 0.0f)
-                contact_linear_viscous<TP>(P, F, T, p, vel_a, angvel_a, S.vel[b],
-                                             xyz(S.angvel[b]), ra, rb, x_ab, len, delta_ab,
-                                             P.kappa);
+                contact_linear_viscous<TP>(P, F, T, p, vel_a, angvel_a, S.vel[b], xyz(S.angvel[b]),
+                                           xa.w, rb, x_ab, len, delta_ab, P.kappa);
             else if (delta_ab < P.db)
-                capillary_exp<TP>(P, F, ra, rb, delta_ab, x_ab, len, P.kappa);
+                capillary_exp<TP>(P, F, xa.w, rb, delta_ab, x_ab, len, P.kappa);
             return true;
-        };
-        if (cnt != NL_OVERFLOW && !(P.db > 0.0 && P.kappa != 0.0)) {
-            for (unsigned j = 0; j < cnt; ++j) {
-                uint32_t e = S.nl[(size_t)j * np + k];
-                uint32_t c = e >> 28;
-                int sx = (c & 1) ? 1 : ((c & 2) ? -1 : 0);
-                int sy = (c & 4) ? 1 : ((c & 8) ? -1 : 0);
-                visit(e & 0x0fffffffu, sx, sy);
-            }
-        } else {
-            for_each_cell_candidate(P, S, k, xa, visit);
-        }
+        });
     }
-
-    contact_walls<PREC>(P, S, xa, ra, vel_a, angvel_a, F, T, es_dot, ev_dot, p, out);
+    contact_walls<PREC>(P, S, xa, xa.w, vel_a, angvel_a, F, T, es_dot, ev_dot, p, out);
     return true;
 }
 
@@ -619,21 +869,25 @@ __device__ __forceinline__ void nl_build_particle(const DevParams &P, const DevS
 #ifndef SPHB_CONTACT_MINB
 #define SPHB_CONTACT_MINB 6
 #endif
-// threads per block of the per-stage contact kernel
+// threads per block of the per-stage contact kernels
 #ifndef SPHB_CONTACT_B
 #define SPHB_CONTACT_B 128
 #endif
-// Contact search and forces of the per-stage path (after k_nl_build).
+// Contact search and forces of the per-stage path (after k_resort); each
+// warp takes pw particles.
 template <int PREC, int MODEL>
-__global__ void __launch_bounds__(SPHB_CONTACT_B, SPHB_CONTACT_MINB) k_contacts(DevParams P, DevState S)
+__global__ void __launch_bounds__(SPHB_CONTACT_B, SPHB_CONTACT_MINB)
+k_contacts(DevParams P, DevState S, unsigned pw)
 {
-    extern __shared__ uint32_t srow[];   // blockDim * nc slot partners
-    const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k == 0 && S.ctl->nl_rebuild) S.ctl->nl_rebuild = 0;  // k_resort has rebuilt the lists
-    if (S.ctl->err || k >= P.np) return;
+    extern __shared__ __align__(16) unsigned char contact_smem[];
+    const unsigned warp = threadIdx.x >> 5, k0 = (blockIdx.x * (blockDim.x >> 5) + warp) * pw;
+    if (k0 == 0 && threadIdx.x == 0 && S.ctl->nl_rebuild) S.ctl->nl_rebuild = 0;  // k_resort has rebuilt the lists
+    // one lane's view decides for the warp: another block may raise it now
+    if (k0 >= P.np || __shfl_sync(0xffffffffu, *(volatile int *)&S.ctl->err, 0)) return;
+    const WarpScratch W = contact_warp_scratch<PREC, MODEL>(contact_smem, warp, P.nc);
     ContactOut c;
-    if (!contact_particle<PREC, MODEL>(P, S, k, srow, blockDim.x, threadIdx.x, c)) return;
-    contact_writeback(P, S, k, c);
+    if (!contact_warp<PREC, MODEL>(P, S, k0, pw, W, c)) return;
+    contact_writeback(P, S, k0 + (threadIdx.x & 31u), c);
 }
 
 // Neighbour list of sorted particle k: every candidate closer than
@@ -873,6 +1127,103 @@ __device__ __forceinline__ bool integrate_particle(const DevParams &P, const Dev
                             resort_flag, nl_flag);
 }
 
+// integrate_values for the particles k0 + ip of a warp whose lanes share a
+// particle (pw <= 8: lane = sub * pw + ip, 32 / pw lanes each): lane sub takes
+// component sub & 3 (x, y, z, w) of the translation (sub >> 2 == 0) or of the
+// rotation (1; with four lanes per particle one after the other).  The
+// arithmetic of a component is integrate_values'; what it saves is the chain:
+// the serial form runs some 1200 instructions in one lane, which is most of a
+// small system's step.  `go` marks the lanes whose particle advances; F and T
+// are valid in the owner lanes (sub 0).  For runs without a shear-stress wall.
+__device__ __forceinline__ void integrate_components(const DevParams &P, const DevState &S, unsigned k,
+                                                     unsigned ip, unsigned sub, unsigned pw, bool go,
+                                                     V3 F, V3 T, const StepClock &clk,
+                                                     int *resort_flag, int *nl_flag)
+{
+    constexpr unsigned ALL = 0xffffffffu;
+    const unsigned ax = sub & 3u;
+    const double Fx = __shfl_sync(ALL, F.x, ip), Fy = __shfl_sync(ALL, F.y, ip), Fz = __shfl_sync(ALL, F.z, ip);
+    const double Tx = __shfl_sync(ALL, T.x, ip), Ty = __shfl_sync(ALL, T.y, ip), Tz = __shfl_sync(ALL, T.z, ip);
+    const double dt = P.dt;
+    int cell = 0;
+    bool inside = true;
+    double drift = 0.0;
+    const size_t at = 4 * (size_t)k + ax;   // this component of particle k
+    auto el = [&](double4 *a) -> double & { return reinterpret_cast<double *>(a)[at]; };
+    auto elf = [&](float4 *a) -> float & { return reinterpret_cast<float *>(a)[at]; };
+    for (unsigned part = sub >> 2; go && part < 2u; part += pw == 8u ? 1u : 2u) {
+        const double radius = S.x[k].w, fix = S.vel[k].w;
+        const bool rot = part == 1u;
+        const double m = 4.0 / 3.0 * SPHB_PI * radius * radius * radius * P.rho;
+        const double q0 = rot ? el(S.angpos) : el(S.x), v0 = rot ? el(S.angvel) : el(S.vel);
+        double4 *const acc_a = rot ? S.angacc : S.acc;
+        const double a0 = clk.iter != 0 ? el(acc_a) : 0.0;
+        double q1 = q0, v1 = v0, a = 0.0, sum = 0.0;
+        if (!rot) sum = el(S.xyzsum);
+        if (ax < 3u) {
+            if (!rot) {
+                a = (ax == 0 ? Fx : ax == 1 ? Fy : Fz) / m + P.g[ax];
+            } else {
+                a = (ax == 0 ? Tx : ax == 1 ? Ty : Tz) * 1.0 / (2.0 / 5.0 * m * radius * radius);
+            }
+            if (fix > 0.0001 && fix < 10.0) {
+                if (rot || ax < 2u) a = 0.0;
+                else a -= P.g[2];
+            }
+            if (fix >= 10.0 && (rot ? ax != 1u : ax == 1u)) a = 0.0;
+            if (fix < -0.0001) a = 0.0;
+            if (P.integrator == 3) {
+                const double da = (a - a0) / dt;
+                q1 = q0 + v0 * dt + 0.5 * a * dt * dt + 1.0 / 6.0 * da * dt * dt * dt;
+                v1 = v0 + a * dt + 0.5 * da * dt * dt;
+                sum += v0 * dt + 0.5 * a * dt * dt + 1.0 / 6.0 * da * dt * dt * dt;
+            } else {
+                q1 = q0 + v0 * dt + 0.5 * a * dt * dt;
+                v1 = v0 + a * dt;
+                sum += v0 * dt + 0.5 * a * dt * dt;
+            }
+        }
+        if (!rot && (ax == 0u ? P.periodic == 1 || P.periodic == 2 : ax == 1u && P.periodic == 1)) {
+            if (q1 < P.origo[ax]) q1 += P.L[ax];
+            if (q1 > P.L[ax]) q1 -= P.L[ax];
+        }
+        if (!rot && ax == 0u && fix > 5.0 && fix < 10.0) {
+            // rate-state velocity step (device.cu:2461-2469)
+            if (clk.t_current >= 10.0 && clk.t_current < 15.0 && clk.velocity_state == 1) v1 *= 10.0;
+            else if (clk.t_current >= 15.0 && clk.velocity_state == 2) v1 /= 10.0;
+        }
+        el(acc_a) = a;
+        if (rot) {
+            el(S.angvel_nx) = v1;
+            el(S.angpos) = q1;
+            if (S.vel_f_nx) elf(S.angvel_f_nx) = ax < 3u ? (float)v1 : 0.0f;
+        } else {
+            el(S.xyzsum) = sum;
+            el(S.vel_nx) = v1;
+            el(S.x_nx) = q1;
+            if (S.vel_f_nx) elf(S.vel_f_nx) = (float)v1;
+            if (ax < 3u) {
+                inside = cell_coord(P, q1, (int)ax, cell);
+                drift = q1 - (double)reinterpret_cast<const float *>(S.x_ref)[at];
+            }
+        }
+    }
+    // the owner joins the three translation lanes
+    const int cy = __shfl_down_sync(ALL, cell, pw), cz = __shfl_down_sync(ALL, cell, 2u * pw);
+    const int iy = __shfl_down_sync(ALL, (int)inside, pw), iz = __shfl_down_sync(ALL, (int)inside, 2u * pw);
+    const double dy = __shfl_down_sync(ALL, drift, pw), dz = __shfl_down_sync(ALL, drift, 2u * pw);
+    if (!go || sub != 0u) return;
+    if (!inside || !iy || !iz) {
+        raise_err(S.ctl, DERR_OUTSIDE, (int)S.orig_of[k]);
+        return;
+    }
+    const unsigned c = ((unsigned)cz * P.num[1]) * P.num[0] + (unsigned)cy * P.num[0] + (unsigned)cell;
+    S.cell_new[k] = c;
+    if (c != S.cell_of[k]) *resort_flag = 1;
+    const double lim = 0.45 * P.skin;
+    if (drift * drift + dy * dy + dz * dz > lim * lim) *nl_flag = 1;
+}
+
 // Copies sorted particle k's x / vel / angvel (and their FP32 copies) into
 // the other buffer of the ping-pong pair unchanged: a step that does not
 // integrate k still hands its state on to the next buffer.
@@ -956,52 +1307,67 @@ __device__ __forceinline__ void finish_step(const DevParams &P, const DevState &
     ctl->iter = iter + 1;
 }
 
-// Contacts, forces and integration of sorted particle k (the particle work
-// of k_contacts_integrate).  After a device error (raised by an earlier
-// step, or by this particle's contact search) the particle's state is
-// carried to the other buffer unchanged.
+// Contacts, forces and integration of the particles k0 .. k0 + pw - 1 by one
+// warp, into the other buffer of the x / vel / angvel pair.  Returns false in
+// the lanes that own a particle whose contact search raised an error, and in
+// those that own none.
 template <int PREC, int MODEL>
-__device__ __forceinline__ void contacts_integrate_particle(const DevParams &P, const DevState &S,
-                                                            unsigned k, uint32_t *srow)
+__device__ __forceinline__ bool contacts_integrate_warp(const DevParams &P, const DevState &S, unsigned k0,
+                                                        unsigned pw, const WarpScratch &W,
+                                                        const StepClock &clk, int *resort_flag, int *nl_flag)
 {
+    const unsigned lane = threadIdx.x & 31u;
+    ContactOut c;
+    c.F = c.T = mk3(0.0, 0.0, 0.0);
+    const bool got = contact_warp<PREC, MODEL>(P, S, k0, pw, W, c);
+    if (got) contact_writeback(P, S, k0 + lane, c);
+    if (pw <= 8u) {
+        const unsigned ip = lane & (pw - 1u);
+        integrate_components(P, S, k0 + ip, ip, lane / pw, pw, __shfl_sync(0xffffffffu, (int)got, ip), c.F, c.T,
+                             clk, resort_flag, nl_flag);
+    } else if (got) {
+        integrate_particle(P, S, k0 + lane, make_double4(c.F.x, c.F.y, c.F.z, 0.0f),
+                           make_double4(c.T.x, c.T.y, c.T.z, 0.0f), clk, S.x_nx, S.vel_nx, S.angvel_nx,
+                           S.vel_f_nx, S.angvel_f_nx, resort_flag, nl_flag);
+    }
+    return got;
+}
+
+// The contact stage and the particle integration of one DEM step in one
+// launch, for dry boxes without bonds, fluid or a shear-stress wall (their
+// forces would have to join before the integration).  A warp runs the contact
+// search and forces of its pw particles, the owners write them back and
+// integrate into the other buffer of the x / vel / angvel ping-pong pair
+// (S.x_nx, ...).  Every partner is read from the current buffer, which no
+// thread of this launch writes, so the particles advance exactly as with
+// k_contacts followed by k_integrate.  The cell and list flags of the next
+// step go to DevCtl::resort_next / nl_next; the wall reduction, the wall
+// update and the loop counters follow in k_walls_step.  After a device error
+// (raised by an earlier step, or by the particle's contact search) the
+// particle's state is carried to the other buffer unchanged.
+template <int PREC, int MODEL>
+__global__ void __launch_bounds__(SPHB_CONTACT_B, SPHB_CONTACT_MINB)
+k_contacts_integrate(DevParams P, DevState S, unsigned pw)
+{
+    extern __shared__ __align__(16) unsigned char contact_smem[];
+    const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const unsigned k0 = (blockIdx.x * (blockDim.x >> 5) + warp) * pw, k = k0 + lane;
+    if (k0 >= P.np) return;   // whole warps
+    const bool own = lane < pw && k < P.np;
     DevCtl *ctl = S.ctl;
-    if (ctl->err) {
-        carry_particle(S, k);
+    // one lane's view decides for the warp: another block may raise it now
+    if (__shfl_sync(0xffffffffu, *(volatile int *)&ctl->err, 0)) {
+        if (own) carry_particle(S, k);
         return;
     }
+    const WarpScratch W = contact_warp_scratch<PREC, MODEL>(contact_smem, warp, P.nc);
     StepClock clk;
     clk.iter = ctl->iter;
     clk.t_current = ctl->t_current;
     clk.velocity_state = ctl->velocity_state;
     clk.tau_eff_x = ctl->tau_eff_x;
-    ContactOut c;
-    if (!contact_particle<PREC, MODEL>(P, S, k, srow, blockDim.x, threadIdx.x, c)) {
+    if (!contacts_integrate_warp<PREC, MODEL>(P, S, k0, pw, W, clk, &ctl->resort_next, &ctl->nl_next) && own)
         carry_particle(S, k);
-        return;
-    }
-    contact_writeback(P, S, k, c);
-    integrate_particle(P, S, k, make_double4(c.F.x, c.F.y, c.F.z, 0.0f),
-                       make_double4(c.T.x, c.T.y, c.T.z, 0.0f), clk, S.x_nx, S.vel_nx,
-                       S.angvel_nx, S.vel_f_nx, S.angvel_f_nx, &ctl->resort_next, &ctl->nl_next);
-}
-
-// The contact stage and the particle integration of one DEM step in one
-// launch, for dry boxes without bonds, fluid or a shear-stress wall (their
-// forces would have to join before the integration).  Thread k runs sorted
-// particle k's contact search and forces, writes them back, then integrates
-// it into the other buffer of the x / vel / angvel ping-pong pair
-// (S.x_nx, ...).  Every partner is read from the current buffer, which no
-// thread of this launch writes, so the particles advance exactly as with
-// k_contacts followed by k_integrate.  The cell and list flags of the next
-// step go to DevCtl::resort_next / nl_next; the wall reduction, the wall
-// update and the loop counters follow in k_walls_step.
-template <int PREC, int MODEL>
-__global__ void __launch_bounds__(SPHB_CONTACT_B, SPHB_CONTACT_MINB)
-k_contacts_integrate(DevParams P, DevState S)
-{
-    extern __shared__ uint32_t srow[];   // blockDim * nc slot partners
-    const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < P.np) contacts_integrate_particle<PREC, MODEL>(P, S, k, srow);
 }
 
 }  // namespace sphb

@@ -5,6 +5,7 @@
 // src/CMakeLists.txt:25).  One thread per particle in sorted order.
 #include "dem_device.cuh"
 #include "contacts_staged.cuh"
+#include "contact_launch.cuh"
 #include "dem_launch.h"
 #include "reduce_device.cuh"
 
@@ -346,48 +347,21 @@ cudaError_t launch_contacts(const DevParams &P, const DevState &S, int prec, cud
         else k_contacts_staged<1><<<grid, SPHB_STAGED_B, smem, st>>>(P, S, cap);
         return cudaGetLastError();
     }
-    const unsigned B = SPHB_CONTACT_B;
-    dim3 grid(blocks_for(P.np, B));
-    if (P.contactmodel == 2) {
-        size_t smem = (size_t)B * P.nc * sizeof(uint32_t);
-        static bool attr = false;
-        if (!attr) {
-            int mx = (int)((size_t)B * 64 * sizeof(uint32_t));
-            cudaFuncSetAttribute(k_contacts<0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-            cudaFuncSetAttribute(k_contacts<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-            attr = true;
-        }
-        if (prec == 0) k_contacts<0, 2><<<grid, B, smem, st>>>(P, S);
-        else k_contacts<1, 2><<<grid, B, smem, st>>>(P, S);
-    } else {
-        if (prec == 0) k_contacts<0, 1><<<grid, B, 0, st>>>(P, S);
-        else k_contacts<1, 1><<<grid, B, 0, st>>>(P, S);
-    }
-    return cudaGetLastError();
+    if (P.contactmodel == 2)
+        return prec == 0 ? launch_contact_kernel<0, 2>(k_contacts<0, 2>, P, S, st)
+                         : launch_contact_kernel<1, 2>(k_contacts<1, 2>, P, S, st);
+    return prec == 0 ? launch_contact_kernel<0, 1>(k_contacts<0, 1>, P, S, st)
+                     : launch_contact_kernel<1, 1>(k_contacts<1, 1>, P, S, st);
 }
 
 cudaError_t launch_contacts_integrate(const DevParams &P, const DevState &S, int prec,
                                       cudaStream_t st)
 {
-    if (P.np == 0) return cudaSuccess;
-    const unsigned B = SPHB_CONTACT_B;
-    dim3 grid(blocks_for(P.np, B));
-    if (P.contactmodel == 2) {
-        size_t smem = (size_t)B * P.nc * sizeof(uint32_t);
-        static bool attr = false;
-        if (!attr) {
-            int mx = (int)((size_t)B * 64 * sizeof(uint32_t));
-            cudaFuncSetAttribute(k_contacts_integrate<0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-            cudaFuncSetAttribute(k_contacts_integrate<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-            attr = true;
-        }
-        if (prec == 0) k_contacts_integrate<0, 2><<<grid, B, smem, st>>>(P, S);
-        else k_contacts_integrate<1, 2><<<grid, B, smem, st>>>(P, S);
-    } else {
-        if (prec == 0) k_contacts_integrate<0, 1><<<grid, B, 0, st>>>(P, S);
-        else k_contacts_integrate<1, 1><<<grid, B, 0, st>>>(P, S);
-    }
-    return cudaGetLastError();
+    if (P.contactmodel == 2)
+        return prec == 0 ? launch_contact_kernel<0, 2>(k_contacts_integrate<0, 2>, P, S, st)
+                         : launch_contact_kernel<1, 2>(k_contacts_integrate<1, 2>, P, S, st);
+    return prec == 0 ? launch_contact_kernel<0, 1>(k_contacts_integrate<0, 1>, P, S, st)
+                     : launch_contact_kernel<1, 1>(k_contacts_integrate<1, 1>, P, S, st);
 }
 
 cudaError_t launch_walls_step(const DevParams &P, const DevState &S, cudaStream_t st)

@@ -3,6 +3,7 @@
 // (compiled with FMA contraction, unlike the FP64 kernels).
 #include "dem_device.cuh"
 #include "contacts_staged.cuh"
+#include "contact_launch.cuh"
 #include "dem_launch.h"
 #include "engine_internal.h"
 
@@ -26,42 +27,14 @@ cudaError_t launch_contacts_mixed(const DevParams &P, const DevState &S, cudaStr
         k_contacts_staged<2><<<grid, SPHB_STAGED_B, smem, st>>>(P, S, cap);
         return cudaGetLastError();
     }
-    const unsigned B = SPHB_CONTACT_B;
-    dim3 grid((P.np + B - 1) / B);
-    if (P.contactmodel == 2) {
-        size_t smem = (size_t)B * P.nc * sizeof(uint32_t);
-        static bool attr = false;
-        if (!attr) {
-            cudaFuncSetAttribute(k_contacts<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)((size_t)B * 64 * sizeof(uint32_t)));
-            attr = true;
-        }
-        k_contacts<2, 2><<<grid, B, smem, st>>>(P, S);
-    } else {
-        k_contacts<2, 1><<<grid, B, 0, st>>>(P, S);
-    }
-    return cudaGetLastError();
+    return P.contactmodel == 2 ? launch_contact_kernel<2, 2>(k_contacts<2, 2>, P, S, st)
+                               : launch_contact_kernel<2, 1>(k_contacts<2, 1>, P, S, st);
 }
 
 cudaError_t launch_contacts_integrate_mixed(const DevParams &P, const DevState &S, cudaStream_t st)
 {
-    if (P.np == 0) return cudaSuccess;
-    const unsigned B = SPHB_CONTACT_B;
-    dim3 grid((P.np + B - 1) / B);
-    if (P.contactmodel == 2) {
-        size_t smem = (size_t)B * P.nc * sizeof(uint32_t);
-        static bool attr = false;
-        if (!attr) {
-            cudaFuncSetAttribute(k_contacts_integrate<2, 2>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)((size_t)B * 64 * sizeof(uint32_t)));
-            attr = true;
-        }
-        k_contacts_integrate<2, 2><<<grid, B, smem, st>>>(P, S);
-    } else {
-        k_contacts_integrate<2, 1><<<grid, B, 0, st>>>(P, S);
-    }
-    return cudaGetLastError();
+    return P.contactmodel == 2 ? launch_contact_kernel<2, 2>(k_contacts_integrate<2, 2>, P, S, st)
+                               : launch_contact_kernel<2, 1>(k_contacts_integrate<2, 1>, P, S, st);
 }
 
 int Engine::mixed_init() { return ST_OK; }

@@ -41,6 +41,9 @@ struct DevState {
     // neighbour lists in sorted order: entry j of particle k at nl[j*np + k]
     // = sorted index | periodic shift code << 28
     uint32_t *nl, *nl_count;
+    // slot that the partner of list entry j of particle k last had in k's row
+    // (nl_slot[j*np + k]): a hint, valid only where the row confirms it
+    uint8_t *nl_slot;
     float4 *x_ref;         // position at the last list build
 
     // walls

@@ -63,6 +63,13 @@ public:
     int graph_view = -1;          // state view the graph was captured with
     bool graph_fused = false;     // the graph holds fused per-stage steps
     bool graph_failed = false;
+    // graph of one call of n < graph_steps steps, per state view
+    struct ShortGraph {
+        cudaGraphExec_t exec = nullptr;
+        uint64_t n = 0;
+        bool fused = false;
+    };
+    ShortGraph short_graph[2];
     bool warmed = false;
 
     std::string err;

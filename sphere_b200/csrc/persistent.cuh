@@ -154,14 +154,13 @@ __device__ __forceinline__ bool group_barrier(GroupSync *g, GroupTree *tree, uns
     return ok != 0;
 }
 
-// Dynamic shared memory: the slot rows (NT * nc u32, at least 16 KB so the
-// same space stages the ordered wall-force sum).  NT threads per block,
+// Dynamic shared memory: the warps' contact scratch (contact_warp_bytes, at
+// least 16 KB so the same space stages the ordered wall-force sum).  NT threads per block,
 // MINB resident blocks per SM (register budget 65536 / (NT * MINB)).
 template <int PREC, int MODEL, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_persistent(BatchArgs A)
 {
     extern __shared__ __align__(16) unsigned char dyn[];
-    uint32_t *srow = reinterpret_cast<uint32_t *>(dyn);
     double *stage = reinterpret_cast<double *>(dyn);
     __shared__ BoxRec box;
     __shared__ double cache[256];
@@ -258,14 +257,19 @@ __global__ void __launch_bounds__(NT, MINB) k_persistent(BatchArgs A)
             clk.velocity_state = h.velocity_state;
             clk.tau_eff_x = 0.0;
             int *fr = &pc->flag_resort[iter & 1], *fn = &pc->flag_nl[iter & 1];
-            for (unsigned k = gtid; k < P.np; k += gstride) {
-                if (nl) nl_build_particle(P, S, k);
-                ContactOut c;
-                if (!contact_particle<PREC, MODEL>(P, S, k, srow, B, t, c)) continue;
-                contact_writeback(P, S, k, c);
-                integrate_particle(P, S, k, make_double4(c.F.x, c.F.y, c.F.z, 0.0f),
-                                   make_double4(c.T.x, c.T.y, c.T.z, 0.0f), clk, S.x_nx, S.vel_nx,
-                                   S.angvel_nx, S.vel_f_nx, S.angvel_f_nx, fr, fn);
+            {
+                const unsigned lane = t & 31u, gwarps = gstride >> 5;
+                const unsigned pw = contact_pw(P.np, gwarps);
+                const WarpScratch ws = contact_warp_scratch<PREC, MODEL>(dyn, t >> 5, P.nc);
+                for (unsigned k0 = (gtid >> 5) * pw; k0 < P.np; k0 += gwarps * pw) {
+                    const unsigned k = k0 + lane;
+                    if (nl) {
+                        if (lane < pw && k < P.np) nl_build_particle(P, S, k);
+                        __syncwarp();   // the warp's lanes read the list
+                    }
+                    contacts_integrate_warp<PREC, MODEL>(P, S, k0, pw, ws, clk, fr, fn);
+                    __syncwarp();
+                }
             }
             if (!bar()) return;
             // ---- W: wall-force partials ----

@@ -47,11 +47,12 @@ inline void set_sync_args(BatchArgs &A, unsigned char *sync)
     A.groups = reinterpret_cast<GroupSync *>(sync + kSyncGroupsOff);
 }
 
-// dynamic shared memory of a launch: slot rows, at least the 16 KB stage
+// dynamic shared memory of a launch: the warps' contact scratch, at least the
+// 16 KB stage
 inline size_t persistent_smem(int threads, unsigned nc)
 {
-    size_t rows = (size_t)threads * nc * 4;
-    return rows > 16384 ? rows : 16384;
+    const size_t warps = (size_t)(threads / 32) * contact_warp_bytes<0, 2>(nc);
+    return warps > 16384 ? warps : 16384;
 }
 
 }  // namespace sphb
