@@ -71,8 +71,25 @@ Engine::~Engine()
     for (ShortGraph &g : short_graph)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     for (void *p : allocations) cudaFree(p);
+    cudaFree(query_buf);
     if (host_pinned) cudaFreeHost(host_pinned);
     if (stream) cudaStreamDestroy(stream);
+}
+
+unsigned char *Engine::query_scratch(size_t bytes)
+{
+    if (bytes <= query_bytes) return query_buf;
+    // earlier queries have finished: each waits for its results
+    cudaFree(query_buf);
+    query_buf = nullptr;
+    query_bytes = 0;
+    if (cudaMalloc((void **)&query_buf, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        query_buf = nullptr;
+        return nullptr;
+    }
+    query_bytes = bytes;
+    return query_buf;
 }
 
 int Engine::fail(int code, const std::string &msg)

@@ -3,6 +3,10 @@
 * The contact kernels give a warp 1, 2, 4, ... 32 particles, by the particle
   count: both sides of each boundary, every step path, bit for bit against the
   oracle.
+* The renderer works in tiles of 16 x 16 pixels and groups of 32 spheres: images
+  and particle counts around their multiples, wide ones (the image plane has no
+  height), tall ones (rows repeat), and an eye among the spheres, pixel for pixel
+  against the renderer that tests every sphere.
 """
 import numpy
 import pytest
@@ -45,3 +49,20 @@ def test_particles_per_warp(tmp_path, n, model):
             assert not bad, (k, n, bad)
     for e in engines.values():
         e.close()
+
+
+@pytest.mark.parametrize("n,w,h,scale", [(1, 16, 16, 1.0), (32, 17, 15, 1.0), (33, 1, 33, 1.0), (300, 40, 16, 1.0),
+                                         (300, 15, 47, 1.0), (300, 48, 48, 12.0)])
+def test_render_tiles(n, w, h, scale):
+    import render_oracle as R
+    from sphere_b200.engine import Engine
+    d = configs.settling_lattice(n=n, seed=103, nx=7, ny=7, nz=7, spacing=0.0195)
+    d.radius = d.radius * scale       # 12: spheres around the eye and behind it
+    with Engine(d, precision="faithful") as e:
+        x, vel = e.get("x"), e.get("vel")
+        for method, max_val in ((0, 1.0), (2, 0.02)):
+            img = e.render(method=method, max_val=max_val, width=w, height=h)
+            val = R.method_values(method, x, vel, e.get("angvel"), e.get("xyzsum"), e.get("angpos"), e.get("p"))
+            ref = R.render(x, vel, d.L, w, h, method=method, val=val, max_val=max_val)
+            assert (ref[:, :, :3] != 255).any() or n == 1
+            assert numpy.array_equal(img[:, :, :3], ref[:, :, :3]), (n, w, h, method)
