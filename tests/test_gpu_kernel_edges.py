@@ -7,6 +7,8 @@
   and particle counts around their multiples, wide ones (the image plane has no
   height), tall ones (rows repeat), and an eye among the spheres, pixel for pixel
   against the renderer that tests every sphere.
+* The Darcy iteration keeps one, two or four cells per thread in registers and
+  leaves out those that cannot change.
 """
 import numpy
 import pytest
@@ -64,5 +66,32 @@ def test_render_tiles(n, w, h, scale):
             img = e.render(method=method, max_val=max_val, width=w, height=h)
             val = R.method_values(method, x, vel, e.get("angvel"), e.get("xyzsum"), e.get("angpos"), e.get("p"))
             ref = R.render(x, vel, d.L, w, h, method=method, val=val, max_val=max_val)
-            assert (ref[:, :, :3] != 255).any() or n == 1
+            assert (ref[:, :, :3] != 255).any() or w < 16 or n == 1
             assert numpy.array_equal(img[:, :, :3], ref[:, :, :3]), (n, w, h, method)
+
+
+# cells that change: one, two or four per thread of the solver's 148 x 256
+# threads, and a lid of cells that stay as they are
+@pytest.mark.parametrize("grid,lid", [((8, 8, 9), 2), ((33, 35, 32), 0), ((40, 40, 60), 3), ((40, 40, 80), 0)])
+def test_darcy_cells_per_thread(tmp_path, grid, lid):
+    from sphere_b200.engine import Engine
+    from test_gpu_darcy import RTOL
+    d = configs.settling_lattice(n=300, seed=51, nx=7, ny=7, nz=7, spacing=0.0195, steps=40)
+    d.num = numpy.array(grid, dtype=numpy.uint32)
+    d.L = numpy.array(grid) * 0.024
+    configs.add_top_wall(d, 10e3)
+    d.w_x[0] = (grid[2] - lid) * 0.024 + 0.001
+    d.wmode[0] = 1
+    # viscous enough for the porosity 0.9 of the empty cells
+    configs.init_fluid_darcy(d, mu=2e-3, k_c=3.5e-13, tolerance=1e-7, maxiter=400, bottom_no_flow=True)
+    path = str(tmp_path / "d.bin")
+    binfile.write_bin(d, path)
+    orc = O.Oracle(path, fluid=True)
+    with Engine(path, fluid=True, precision="faithful") as e:
+        for _ in range(3):
+            assert e.step(1) >= 0
+            assert orc.step(1) == 0, orc.error()
+            assert int(e.get("darcy_iters")[0]) == int(orc.get("darcy_nijac_last")[0])
+            for f in ("darcy_p", "darcy_v", "darcy_phi"):
+                a, b = numpy.ravel(e.get(f)), numpy.ravel(orc.get(f))
+                assert numpy.abs(a - b).max() <= RTOL * max(numpy.abs(b).max(), 1e-300), f
