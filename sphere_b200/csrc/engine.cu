@@ -71,25 +71,26 @@ Engine::~Engine()
     for (ShortGraph &g : short_graph)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     for (void *p : allocations) cudaFree(p);
-    cudaFree(query_buf);
+    cudaFree(query_buf[0]);
+    cudaFree(query_buf[1]);
     if (host_pinned) cudaFreeHost(host_pinned);
     if (stream) cudaStreamDestroy(stream);
 }
 
-unsigned char *Engine::query_scratch(size_t bytes)
+unsigned char *Engine::query_scratch(size_t bytes, int which)
 {
-    if (bytes <= query_bytes) return query_buf;
+    if (bytes <= query_bytes[which]) return query_buf[which];
     // earlier queries have finished: each waits for its results
-    cudaFree(query_buf);
-    query_buf = nullptr;
-    query_bytes = 0;
-    if (cudaMalloc((void **)&query_buf, bytes) != cudaSuccess) {
+    cudaFree(query_buf[which]);
+    query_buf[which] = nullptr;
+    query_bytes[which] = 0;
+    if (cudaMalloc((void **)&query_buf[which], bytes) != cudaSuccess) {
         cudaGetLastError();
-        query_buf = nullptr;
+        query_buf[which] = nullptr;
         return nullptr;
     }
-    query_bytes = bytes;
-    return query_buf;
+    query_bytes[which] = bytes;
+    return query_buf[which];
 }
 
 int Engine::fail(int code, const std::string &msg)

@@ -95,13 +95,13 @@ public:
     int fail(int code, const std::string &msg);
     int cuda_fail(cudaError_t e, const char *where);
     template <class T> T *dalloc(size_t n);
-    // Device scratch of the query calls (diagnostics, images): one buffer per
+    // Device scratch of the query calls (diagnostics, images): two buffers per
     // engine, grown to the largest request and released with the engine.  The
     // calls of one handle run one after the other on its stream, so they share
-    // it.  Null when it cannot be allocated.
-    unsigned char *query_scratch(size_t bytes);
-    unsigned char *query_buf = nullptr;
-    size_t query_bytes = 0;
+    // them.  Null when it cannot be allocated.
+    unsigned char *query_scratch(size_t bytes, int which = 0);
+    unsigned char *query_buf[2] = {nullptr, nullptr};
+    size_t query_bytes[2] = {0, 0};
 
     void build_params();
     int allocate_and_upload();

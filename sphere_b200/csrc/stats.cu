@@ -48,31 +48,37 @@ __device__ double block_tree_sum(double v, double *sh)
 // Per-particle energy terms of sim.energy() (python/sphere.py:4327-4358):
 // m = 4/3 pi r^3 rho evaluated as (4/3 * pi) * r**3 * rho;
 // pot = m |g| z; kin = 1/2 m sqrt(v.v)^2; rot = 1/2 2/5 m r^2 sqrt(w.w)^2.
-__global__ void __launch_bounds__(STAT_THREADS) k_energy_partials(DevParams P, DevState S,
+// Block sums of the term `which` alone: a query reads the arrays its term needs.
+__global__ void __launch_bounds__(STAT_THREADS) k_energy_partials(DevParams P, DevState S, int which,
                                                                   double *part)
 {
     __shared__ double sh[STAT_THREADS];
     const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
-    double t[NSUMS] = {0, 0, 0, 0, 0, 0, 0};
+    double t = 0.0;
     if (k < P.np) {
-        const double4 x = S.x[k], v = S.vel[k], w = S.angvel[k];
-        const double r = x.w;
-        const double m = 4.0 / 3.0 * PI_FULL * pow(r, 3.0) * P.rho;
-        const double gabs = sqrt(P.g[0] * P.g[0] + P.g[1] * P.g[1] + P.g[2] * P.g[2]);
-        t[0] = m * gabs * x.z;
-        const double sv = sqrt(v.x * v.x + v.y * v.y + v.z * v.z);
-        t[1] = 0.5 * m * (sv * sv);
-        const double sw = sqrt(w.x * w.x + w.y * w.y + w.z * w.z);
-        t[2] = 0.5 * 2.0 / 5.0 * m * (r * r) * (sw * sw);
-        t[3] = S.es[k];
-        t[4] = S.es_dot[k];
-        t[5] = S.ev[k];
-        t[6] = S.ev_dot[k];
+        if (which < 3) {
+            const double4 x = S.x[k];
+            const double r = x.w;
+            const double m = 4.0 / 3.0 * PI_FULL * pow(r, 3.0) * P.rho;
+            if (which == 0) {
+                const double gabs = sqrt(P.g[0] * P.g[0] + P.g[1] * P.g[1] + P.g[2] * P.g[2]);
+                t = m * gabs * x.z;
+            } else if (which == 1) {
+                const double4 v = S.vel[k];
+                const double sv = sqrt(v.x * v.x + v.y * v.y + v.z * v.z);
+                t = 0.5 * m * (sv * sv);
+            } else {
+                const double4 w = S.angvel[k];
+                const double sw = sqrt(w.x * w.x + w.y * w.y + w.z * w.z);
+                t = 0.5 * 2.0 / 5.0 * m * (r * r) * (sw * sw);
+            }
+        } else {
+            const double *a = which == 3 ? S.es : which == 4 ? S.es_dot : which == 5 ? S.ev : S.ev_dot;
+            t = a[k];
+        }
     }
-    for (int s = 0; s < NSUMS; ++s) {
-        double b = block_tree_sum(t[s], sh);
-        if (threadIdx.x == 0) part[(size_t)blockIdx.x * NSUMS + s] = b;
-    }
+    const double b = block_tree_sum(t, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = b;
 }
 
 // Bond energy terms of sim.energy('bondpot') (python/sphere.py:4360-4376):
@@ -155,125 +161,161 @@ __global__ void __launch_bounds__(STAT_THREADS) k_porosity_partials(DevParams P,
 
 // ---- overlap list (src/sphere.cpp:677-725) ----
 
-// Largest radius, as the bit pattern of a positive double (ordered like u64).
-__global__ void k_rmax(DevParams P, DevState S, unsigned long long *out)
+// Cell of each sorted position from its current coordinates, counts per cell,
+// and the largest radius (as the bit pattern of a positive double, ordered
+// like u64).  Particles outside the grid are counted in *outside (the engine's
+// error flag is left alone).
+__global__ void k_ov_hash(DevParams P, DevState S, uint32_t *key, uint32_t *cnt, uint32_t *outside,
+                          unsigned long long *rmax)
 {
     const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < P.np) atomicMax(out, (unsigned long long)__double_as_longlong(S.x[k].w));
-}
-
-// Cell of each ORIGINAL index from its current position; counts per cell.
-// Particles outside the grid are counted in *outside (the engine's error
-// flag is left alone).
-__global__ void k_ov_hash(DevParams P, DevState S, uint32_t *key, uint32_t *cnt, uint32_t *outside)
-{
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.np) return;
-    const double4 x = S.x[S.pos_of[i]];
-    int c[3];
-    if (!cell_coord(P, x.x, 0, c[0]) || !cell_coord(P, x.y, 1, c[1]) || !cell_coord(P, x.z, 2, c[2])) {
-        atomicAdd(outside, 1u);
-        key[i] = 0xffffffffu;
-        return;
-    }
-    const uint32_t kk = ((uint32_t)c[2] * P.num[1] + (uint32_t)c[1]) * P.num[0] + (uint32_t)c[0];
-    key[i] = kk;
-    atomicAdd(cnt + kk, 1u);
-}
-
-// Exclusive scan of n counts by one block (diagnostic sizes; each thread
-// owns one contiguous chunk).  out[n] = total.
-__global__ void __launch_bounds__(1024) k_scan_1block(const uint32_t *in, uint32_t *out, uint32_t n)
-{
-    __shared__ uint32_t tot[1024];
-    const uint32_t T = blockDim.x, t = threadIdx.x;
-    const uint32_t chunk = (n + T - 1) / T;
-    const uint32_t b = min(n, t * chunk), e = min(n, b + chunk);
-    uint32_t s = 0;
-    for (uint32_t i = b; i < e; ++i) s += in[i];
-    tot[t] = s;
-    __syncthreads();
-    if (t == 0) {
-        uint32_t run = 0;
-        for (uint32_t i = 0; i < T; ++i) {
-            uint32_t v = tot[i];
-            tot[i] = run;
-            run += v;
+    unsigned long long r = 0;
+    if (k < P.np) {
+        const double4 x = S.x[k];
+        r = (unsigned long long)__double_as_longlong(x.w);
+        int c[3];
+        if (!cell_coord(P, x.x, 0, c[0]) || !cell_coord(P, x.y, 1, c[1]) || !cell_coord(P, x.z, 2, c[2])) {
+            atomicAdd(outside, 1u);
+            key[k] = 0xffffffffu;
+        } else {
+            const uint32_t kk = ((uint32_t)c[2] * P.num[1] + (uint32_t)c[1]) * P.num[0] + (uint32_t)c[0];
+            key[k] = kk;
+            atomicAdd(cnt + kk, 1u);
         }
-        out[n] = run;
+    }
+    for (int o = 16; o > 0; o >>= 1) r = max(r, __shfl_xor_sync(0xffffffffu, r, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(rmax, r);
+}
+
+// Exclusive scan of n counts: each block scans its 1024 (sums to tot), one
+// block scans the sums, each block adds its own.  out[n] = total.
+constexpr uint32_t kScanBlock = 1024;
+
+__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *warp_sum, uint32_t &total)
+{
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    uint32_t x = v;
+    for (uint32_t d = 1; d < 32u; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= d) x += y;
+    }
+    if (lane == 31u) warp_sum[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        uint32_t s = warp_sum[lane];
+        for (uint32_t d = 1; d < 32u; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, s, d);
+            if (lane >= d) s += y;
+        }
+        warp_sum[lane] = s;
     }
     __syncthreads();
-    uint32_t run = tot[t];
-    for (uint32_t i = b; i < e; ++i) {
-        uint32_t v = in[i];
-        out[i] = run;
-        run += v;
+    const uint32_t before = w ? warp_sum[w - 1] : 0u;
+    total = warp_sum[31];
+    __syncthreads();
+    return before + x - v;
+}
+
+__global__ void __launch_bounds__(kScanBlock) k_scan_blocks(const uint32_t *in, uint32_t *out, uint32_t n,
+                                                            uint32_t *tot)
+{
+    __shared__ uint32_t ws[32];
+    const uint32_t i = blockIdx.x * kScanBlock + threadIdx.x;
+    uint32_t total;
+    const uint32_t e = block_exclusive(i < n ? in[i] : 0u, ws, total);
+    if (i < n) out[i] = e;
+    if (threadIdx.x == 0) tot[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kScanBlock) k_scan_tops(uint32_t *tot, uint32_t nb, uint32_t *all)
+{
+    __shared__ uint32_t ws[32];
+    uint32_t run = 0;
+    for (uint32_t base = 0; base < nb; base += kScanBlock) {
+        const uint32_t i = base + threadIdx.x;
+        uint32_t total;
+        const uint32_t e = block_exclusive(i < nb ? tot[i] : 0u, ws, total);
+        if (i < nb) tot[i] = run + e;
+        run += total;
     }
+    if (threadIdx.x == 0) *all = run;
+}
+
+__global__ void __launch_bounds__(kScanBlock) k_scan_add(uint32_t *out, uint32_t n, const uint32_t *tot)
+{
+    const uint32_t i = blockIdx.x * kScanBlock + threadIdx.x;
+    if (i < n) out[i] += tot[blockIdx.x];
 }
 
 __global__ void k_ov_fill(DevParams P, const uint32_t *key, const uint32_t *start, uint32_t *fill,
                           uint32_t *list)
 {
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.np || key[i] == 0xffffffffu) return;
-    list[start[key[i]] + atomicAdd(fill + key[i], 1u)] = i;
+    const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= P.np || key[k] == 0xffffffffu) return;
+    list[start[key[k]] + atomicAdd(fill + key[k], 1u)] = k;
 }
 
 // Pairs (i, j > i) of ORIGINAL indices with negative separation
 // |x_j - x_i| - (r_i + r_j) whose fixvel flags are both zero
 // (src/sphere.cpp:690-722), among cells within `reach` of i's cell (no
 // periodic images, like the reference).  PASS 0 counts, PASS 1 writes the
-// pairs of i from out_off[i] on and then orders them by j.
+// pairs of i from out_off[i] on and then orders them by j.  Threads take the
+// particles in sorted order, so neighbouring threads read the same cells, and
+// the squared distance settles the pairs that are clearly apart.
 template <int PASS>
 __global__ void __launch_bounds__(STAT_THREADS) k_ov_search(DevParams P, DevState S, const uint32_t *key,
                                                              const uint32_t *start, const uint32_t *list,
                                                              int3 reach, uint32_t *count,
-                                                             const uint32_t *out_off, uint32_t *out_j,
+                                                             const uint32_t *out_off, uint2 *out_ij,
                                                              double *out_d)
 {
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.np || key[i] == 0xffffffffu) return;
-    const double4 xi = S.x[S.pos_of[i]];
-    const double4 vi = S.vel[S.pos_of[i]];
+    const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= P.np || key[k] == 0xffffffffu) return;
+    const uint32_t i = S.orig_of[k];
+    const double4 xi = S.x[k];
     uint32_t n = 0;
-    if (vi.w == 0.0) {
-        const uint32_t kk = key[i];
+    if (S.vel[k].w == 0.0) {
+        const uint32_t kk = key[k];
         const int cx = (int)(kk % P.num[0]), cy = (int)((kk / P.num[0]) % P.num[1]),
                   cz = (int)(kk / (P.num[0] * P.num[1]));
         const uint32_t base = PASS ? out_off[i] : 0u;
         for (int z = max(0, cz - reach.z); z <= min((int)P.num[2] - 1, cz + reach.z); ++z)
-            for (int y = max(0, cy - reach.y); y <= min((int)P.num[1] - 1, cy + reach.y); ++y)
-                for (int x = max(0, cx - reach.x); x <= min((int)P.num[0] - 1, cx + reach.x); ++x) {
-                    const uint32_t c = ((uint32_t)z * P.num[1] + (uint32_t)y) * P.num[0] + (uint32_t)x;
-                    for (uint32_t q = start[c]; q < start[c + 1]; ++q) {
-                        const uint32_t j = list[q];
-                        if (j <= i) continue;
-                        const uint32_t pj = S.pos_of[j];
-                        const double4 xj = S.x[pj];
-                        const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-                        const double len = sqrt(dx * dx + dy * dy + dz * dz);
-                        const double delta = len - (xi.w + xj.w);
-                        if (delta < 0.0 && S.vel[pj].w == 0.0) {
-                            if (PASS) {
-                                out_j[base + n] = j;
-                                out_d[base + n] = delta;
-                            }
-                            ++n;
+            for (int y = max(0, cy - reach.y); y <= min((int)P.num[1] - 1, cy + reach.y); ++y) {
+                // a row of cells is one range of the list
+                const uint32_t row = ((uint32_t)z * P.num[1] + (uint32_t)y) * P.num[0];
+                const uint32_t q1 = start[row + (uint32_t)min((int)P.num[0] - 1, cx + reach.x) + 1u];
+                for (uint32_t q = start[row + (uint32_t)max(0, cx - reach.x)]; q < q1; ++q) {
+                    const uint32_t pj = list[q];
+                    const double4 xj = S.x[pj];
+                    const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
+                    const double d2 = dx * dx + dy * dy + dz * dz, rs = xi.w + xj.w;
+                    // the rounded root of more than (1 + 1e-12) rs^2 exceeds rs
+                    if (d2 > rs * rs * (1.0 + 1e-12) && d2 > 1e-200) continue;
+                    const uint32_t j = S.orig_of[pj];
+                    if (j <= i) continue;
+                    const double len = sqrt(d2);
+                    const double delta = len - rs;
+                    if (delta < 0.0 && S.vel[pj].w == 0.0) {
+                        if (PASS) {
+                            out_ij[base + n] = make_uint2(i, j);
+                            out_d[base + n] = delta;
                         }
+                        ++n;
                     }
                 }
+            }
         if (PASS) {
             // insertion sort of this particle's segment by j
             for (uint32_t a = 1; a < n; ++a) {
-                const uint32_t jj = out_j[base + a];
+                const uint32_t jj = out_ij[base + a].y;
                 const double dd = out_d[base + a];
                 uint32_t b = a;
-                while (b > 0 && out_j[base + b - 1] > jj) {
-                    out_j[base + b] = out_j[base + b - 1];
+                while (b > 0 && out_ij[base + b - 1].y > jj) {
+                    out_ij[base + b].y = out_ij[base + b - 1].y;
                     out_d[base + b] = out_d[base + b - 1];
                     --b;
                 }
-                out_j[base + b] = jj;
+                out_ij[base + b].y = jj;
                 out_d[base + b] = dd;
             }
         }
@@ -281,19 +323,25 @@ __global__ void __launch_bounds__(STAT_THREADS) k_ov_search(DevParams P, DevStat
     if (!PASS) count[i] = n;
 }
 
-// RAII device scratch for one diagnostic call.
-struct Scratch {
-    std::vector<void *> p;
+// Exclusive scan of n counts into out[0..n], with (n + 1023) / 1024 words of
+// scratch.
+void scan_counts(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *tot, cudaStream_t st)
+{
+    const uint32_t nb = (n + kScanBlock - 1) / kScanBlock;
+    k_scan_blocks<<<nb, kScanBlock, 0, st>>>(in, out, n, tot);
+    k_scan_tops<<<1, kScanBlock, 0, st>>>(tot, nb, out + n);
+    k_scan_add<<<nb, kScanBlock, 0, st>>>(out, n, tot);
+}
+
+// Carves arrays from one buffer: first pass (null base) adds up the bytes.
+struct Carve {
+    unsigned char *base;
+    size_t off = 0;
     template <class T> T *get(size_t n)
     {
-        void *q = nullptr;
-        if (cudaMalloc(&q, (n ? n : 1) * sizeof(T)) != cudaSuccess) return nullptr;
-        p.push_back(q);
-        return (T *)q;
-    }
-    ~Scratch()
-    {
-        for (void *q : p) cudaFree(q);
+        T *p = base ? reinterpret_cast<T *>(base + off) : nullptr;
+        off += (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~(size_t)255;
+        return p;
     }
 };
 
@@ -311,21 +359,20 @@ int Engine::energy(const char *method, double *out)
     if (which < 0 && !bond) return fail(ST_ARG, std::string("Unknown energy() method \"") + method + "\"");
     int rc = poll_errors("energy");
     if (rc < 0 && rc != ST_OUTSIDE && rc != ST_CAPACITY) return rc;
-    Scratch sc;
     cudaError_t e = cudaSuccess;
     if (!bond) {
         const unsigned nb = blocks_of(hs.np, STAT_THREADS);
-        double *part = sc.get<double>((size_t)nb * NSUMS);
+        double *part = (double *)query_scratch(std::max<size_t>(nb, 1) * 8);
         if (!part) return fail(ST_CUDA, "energy: out of device memory");
-        if (nb) k_energy_partials<<<nb, STAT_THREADS, 0, stream>>>(P, S, part);
-        std::vector<double> h((size_t)nb * NSUMS);
+        if (nb) k_energy_partials<<<nb, STAT_THREADS, 0, stream>>>(P, S, which, part);
+        std::vector<double> h(nb);
         e = cudaGetLastError();
         if (e == cudaSuccess && nb)
             e = cudaMemcpyAsync(h.data(), part, h.size() * 8, cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return cuda_fail(e, "energy");
         double acc = 0.0;
-        for (unsigned b = 0; b < nb; ++b) acc += h[(size_t)b * NSUMS + which];
+        for (unsigned b = 0; b < nb; ++b) acc += h[b];
         *out = acc;
         return ST_OK;
     }
@@ -342,7 +389,7 @@ int Engine::energy(const char *method, double *out)
     for (uint32_t v : bonds)
         if (v >= hs.np) return fail(ST_ARG, "energy: a bond refers to a particle index beyond np");
     const unsigned nb = blocks_of(hs.nb0, STAT_THREADS);
-    double *part = sc.get<double>((size_t)nb * 6);
+    double *part = (double *)query_scratch((size_t)nb * 6 * 8);
     if (!part) return fail(ST_CUDA, "energy: out of device memory");
     k_bond_partials<<<nb, STAT_THREADS, 0, stream>>>(P, S, part);
     std::vector<double> h((size_t)nb * 6);
@@ -390,9 +437,8 @@ int Engine::porosity_profile(int z_slices, double *z_pos, double *porosity)
     const double V_slice = h_slice * hs.L[0] * hs.L[1];
     const unsigned nb = blocks_of(hs.np, STAT_THREADS);
     std::vector<double> h((size_t)nb * z_slices);
-    Scratch sc;
     if (nb) {
-        double *part = sc.get<double>(h.size());
+        double *part = (double *)query_scratch(h.size() * 8);
         if (!part) return fail(ST_CUDA, "porosity: out of device memory");
         k_porosity_partials<<<dim3(nb, (unsigned)z_slices), STAT_THREADS, 0, stream>>>(P, S, h_slice, part);
         e = cudaGetLastError();
@@ -418,23 +464,35 @@ int Engine::overlaps(uint32_t *pairs, double *delta, uint64_t cap, uint64_t *cou
     if (rc < 0) return rc;
     const size_t n = hs.np, nc = hs.ncells();
     if (n == 0) return ST_OK;
-    Scratch sc;
-    unsigned long long *rmax_bits = sc.get<unsigned long long>(1);
-    uint32_t *outside = sc.get<uint32_t>(1);
-    uint32_t *key = sc.get<uint32_t>(n), *cnt = sc.get<uint32_t>(nc), *start = sc.get<uint32_t>(nc + 1),
-             *fill = sc.get<uint32_t>(nc), *list = sc.get<uint32_t>(n), *pc = sc.get<uint32_t>(n),
-             *off = sc.get<uint32_t>(n + 1);
-    if (!rmax_bits || !outside || !key || !cnt || !start || !fill || !list || !pc || !off)
-        return fail(ST_CUDA, "overlaps: out of device memory");
+    unsigned long long *rmax_bits = nullptr;
+    uint32_t *outside = nullptr, *cnt = nullptr, *fill = nullptr, *key = nullptr, *start = nullptr, *list = nullptr,
+             *pc = nullptr, *off = nullptr, *tot = nullptr;
+    size_t zeroed = 0;
+    Carve sc{nullptr};
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass) {
+            unsigned char *ws = query_scratch(sc.off);
+            if (!ws) return fail(ST_CUDA, "overlaps: out of device memory");
+            sc = Carve{ws};
+        }
+        rmax_bits = sc.get<unsigned long long>(1);
+        outside = sc.get<uint32_t>(1);
+        cnt = sc.get<uint32_t>(nc);
+        fill = sc.get<uint32_t>(nc);
+        zeroed = sc.off;
+        key = sc.get<uint32_t>(n);
+        start = sc.get<uint32_t>(nc + 1);
+        list = sc.get<uint32_t>(n);
+        pc = sc.get<uint32_t>(n);
+        off = sc.get<uint32_t>(n + 1);
+        tot = sc.get<uint32_t>(std::max(n, nc) / kScanBlock + 1);
+    }
     const unsigned nb = blocks_of(n, STAT_THREADS);
-    cudaError_t e = cudaMemsetAsync(rmax_bits, 0, 8, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(outside, 0, 4, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, nc * 4, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(fill, 0, nc * 4, stream);
+    // the counters are the first arrays
+    cudaError_t e = cudaMemsetAsync(rmax_bits, 0, zeroed, stream);
     if (e != cudaSuccess) return cuda_fail(e, "overlaps");
-    k_rmax<<<nb, STAT_THREADS, 0, stream>>>(P, S, rmax_bits);
-    k_ov_hash<<<nb, STAT_THREADS, 0, stream>>>(P, S, key, cnt, outside);
-    k_scan_1block<<<1, 1024, 0, stream>>>(cnt, start, (uint32_t)nc);
+    k_ov_hash<<<nb, STAT_THREADS, 0, stream>>>(P, S, key, cnt, outside, rmax_bits);
+    scan_counts(cnt, start, (uint32_t)nc, tot, stream);
     k_ov_fill<<<nb, STAT_THREADS, 0, stream>>>(P, key, start, fill, list);
     unsigned long long bits = 0;
     uint32_t nout = 0;
@@ -456,7 +514,7 @@ int Engine::overlaps(uint32_t *pairs, double *delta, uint64_t cap, uint64_t *cou
     const int3 r3 = make_int3(reach[0], reach[1], reach[2]);
     k_ov_search<0><<<nb, STAT_THREADS, 0, stream>>>(P, S, key, start, list, r3, pc, nullptr, nullptr,
                                                     nullptr);
-    k_scan_1block<<<1, 1024, 0, stream>>>(pc, off, (uint32_t)n);
+    scan_counts(pc, off, (uint32_t)n, tot, stream);
     uint32_t total = 0;
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(&total, off + n, 4, cudaMemcpyDeviceToHost, stream);
@@ -466,22 +524,17 @@ int Engine::overlaps(uint32_t *pairs, double *delta, uint64_t cap, uint64_t *cou
     if (!pairs && !delta) return ST_OK;
     if (!pairs || !delta || cap < total) return fail(ST_ARG, "overlaps: output buffers hold fewer pairs than found");
     if (total == 0) return ST_OK;
-    uint32_t *oj = sc.get<uint32_t>(total);
-    double *od = sc.get<double>(total);
-    if (!oj || !od) return fail(ST_CUDA, "overlaps: out of device memory");
-    k_ov_search<1><<<nb, STAT_THREADS, 0, stream>>>(P, S, key, start, list, r3, nullptr, off, oj, od);
-    std::vector<uint32_t> hj(total), hoff(n + 1);
+    // the pairs have their own buffer: the lists above are still read
+    unsigned char *pb = query_scratch((size_t)total * 16 + 256, 1);
+    if (!pb) return fail(ST_CUDA, "overlaps: out of device memory");
+    double *od = (double *)pb;
+    uint2 *oij = (uint2 *)(pb + (((size_t)total * 8 + 255) & ~(size_t)255));
+    k_ov_search<1><<<nb, STAT_THREADS, 0, stream>>>(P, S, key, start, list, r3, nullptr, off, oij, od);
     e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hj.data(), oj, total * 4ull, cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(pairs, oij, total * 8ull, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(delta, od, total * 8ull, cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hoff.data(), off, (n + 1) * 4, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return cuda_fail(e, "overlaps");
-    for (size_t i = 0; i < n; ++i)
-        for (uint32_t q = hoff[i]; q < hoff[i + 1]; ++q) {
-            pairs[2 * (size_t)q] = (uint32_t)i;
-            pairs[2 * (size_t)q + 1] = hj[q];
-        }
     return ST_OK;
 }
 
