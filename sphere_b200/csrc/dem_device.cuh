@@ -6,6 +6,7 @@
 
 #include "dem_state.h"
 #include "reduce_device.cuh"
+#include "resort_device.cuh"
 
 namespace sphb {
 
@@ -547,9 +548,15 @@ __device__ __forceinline__ bool touches(const DevParams &P, const double4 &xa, c
 // 14 us, and 54 and 18 us for the whole step).
 // PREC 0: faithful FP64, 1: FP64, 2: mixed (FP64 overlap, FP32 contact law,
 // FP64 accumulation).
-template <int PREC, int MODEL>
+// before_walls() runs in all lanes once the contacts are done and before the
+// walls are read.
+struct WallsReady {
+    __device__ __forceinline__ void operator()() const {}
+};
+template <int PREC, int MODEL, class Before = WallsReady>
 __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState &S, unsigned k0,
-                                             unsigned pw, const WarpScratch &W, ContactOut &out)
+                                             unsigned pw, const WarpScratch &W, ContactOut &out,
+                                             Before &&before_walls = Before())
 {
     constexpr int TP = PREC == 2 ? 1 : PREC;  // precision of overlap tests
     constexpr unsigned ALL = 0xffffffffu;
@@ -816,6 +823,7 @@ __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState 
         }
         __syncwarp();
     }
+    before_walls();
     if (!ok) return false;
     const double4 vel_a = S.vel[k];
     const V3 angvel_a = xyz(S.angvel[k]);
@@ -839,6 +847,43 @@ __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState 
     }
     contact_walls<PREC>(P, S, xa, xa.w, vel_a, angvel_a, F, T, es_dot, ev_dot, p, out);
     return true;
+}
+
+// Adds the bond forces of the particle with original index o in increasing
+// bond order (k_bonds' results; a broken bond adds zeros, and a sum that
+// started at +0 keeps its bits).  bond_list entries are (bond index << 1) | (1
+// if the particle is the bond's second).  Returns whether it has bonds.
+__device__ __forceinline__ bool add_bonds(const DevState &S, unsigned o, V3 &F, V3 &T)
+{
+    const unsigned b0 = S.bond_ptr[o], b1 = S.bond_ptr[o + 1];
+    for (unsigned j0 = b0; j0 < b1; j0 += 4u) {
+        // four bonds' loads in flight
+        unsigned e[4];
+        double2 v[4][3];
+#pragma unroll
+        for (unsigned q = 0; q < 4; ++q) e[q] = j0 + q < b1 ? S.bond_list[j0 + q] : 0u;
+#pragma unroll
+        for (unsigned q = 0; q < 4; ++q)
+            if (j0 + q < b1) {
+                const double2 *ft = S.bond_ft + 3 * (size_t)(e[q] >> 1);
+                v[q][0] = ft[0];
+                v[q][1] = ft[1];
+                v[q][2] = ft[2];
+            }
+#pragma unroll
+        for (unsigned q = 0; q < 4; ++q)
+            if (j0 + q < b1) {
+                const V3 f = mk3(v[q][0].x, v[q][0].y, v[q][1].x), t = mk3(v[q][1].y, v[q][2].x, v[q][2].y);
+                if ((e[q] & 1u) == 0) {
+                    F = add3(F, f);
+                    T = sub3(T, t);
+                } else {
+                    F = sub3(F, f);
+                    T = add3(T, t);
+                }
+            }
+    }
+    return b0 != b1;
 }
 
 // Write-back of one particle's contact results (contactsearch.cuh:706-724).
@@ -922,6 +967,13 @@ struct StepClock {
     double tau_eff_x;
 };
 
+// Where an integration step reports what the next step has to do first, and
+// the value it writes there.
+struct StepFlags {
+    int *resort, *nl;
+    int value;
+};
+
 // The inputs of one particle's integration step (its state before the step
 // and the forces of the step).
 struct IntegrateIn {
@@ -937,15 +989,14 @@ struct IntegrateIn {
 // angvel (and their FP32 copies when vel_f_out is set) to the *_out arrays
 // -- S's own arrays for the in-place kernel, the other buffer of a ping-pong
 // pair for the fused step -- and acc, angacc, angpos, xyzsum, cell_new to S.
-// Raises *resort_flag when the cell changed and *nl_flag when the particle
+// Raises flags.resort when the cell changed and flags.nl when the particle
 // left its neighbour-list skin.  Returns false after raising an outside-grid
 // error.
 __device__ __forceinline__ bool integrate_values(const DevParams &P, const DevState &S, unsigned k,
                                                  const IntegrateIn &in, const StepClock &clk,
                                                  double4 *x_out, double4 *vel_out,
                                                  double4 *angvel_out, float4 *vel_f_out,
-                                                 float4 *angvel_f_out, int *resort_flag,
-                                                 int *nl_flag)
+                                                 float4 *angvel_f_out, StepFlags flags)
 {
     const long long iter = clk.iter;
     const double t_current = clk.t_current;
@@ -1088,13 +1139,13 @@ __device__ __forceinline__ bool integrate_values(const DevParams &P, const DevSt
     }
     unsigned c = ((unsigned)iz * P.num[1]) * P.num[0] + (unsigned)iy * P.num[0] + (unsigned)ix;
     S.cell_new[k] = c;
-    if (c != in.cell) *resort_flag = 1;
+    if (c != in.cell) *flags.resort = flags.value;
     // neighbour lists stay exact while every particle is within 0.45 skin
     // of its position at the build
     const float4 xr = in.x_ref;
     double ddx = x_new.x - (double)xr.x, ddy = x_new.y - (double)xr.y, ddz = x_new.z - (double)xr.z;
     double lim = 0.45 * P.skin;
-    if (ddx * ddx + ddy * ddy + ddz * ddz > lim * lim) *nl_flag = 1;
+    if (ddx * ddx + ddy * ddy + ddz * ddz > lim * lim) *flags.nl = flags.value;
     return true;
 }
 
@@ -1104,8 +1155,7 @@ __device__ __forceinline__ bool integrate_particle(const DevParams &P, const Dev
                                                    double4 force, double4 torque, const StepClock &clk,
                                                    double4 *x_out, double4 *vel_out,
                                                    double4 *angvel_out, float4 *vel_f_out,
-                                                   float4 *angvel_f_out, int *resort_flag,
-                                                   int *nl_flag)
+                                                   float4 *angvel_f_out, StepFlags flags)
 {
     IntegrateIn in;
     in.force = force;
@@ -1124,7 +1174,7 @@ __device__ __forceinline__ bool integrate_particle(const DevParams &P, const Dev
     in.cell = S.cell_of[k];
     in.x_ref = S.x_ref[k];
     return integrate_values(P, S, k, in, clk, x_out, vel_out, angvel_out, vel_f_out, angvel_f_out,
-                            resort_flag, nl_flag);
+                            flags);
 }
 
 // integrate_values for the particles k0 + ip of a warp whose lanes share a
@@ -1138,7 +1188,7 @@ __device__ __forceinline__ bool integrate_particle(const DevParams &P, const Dev
 __device__ __forceinline__ void integrate_components(const DevParams &P, const DevState &S, unsigned k,
                                                      unsigned ip, unsigned sub, unsigned pw, bool go,
                                                      V3 F, V3 T, const StepClock &clk,
-                                                     int *resort_flag, int *nl_flag)
+                                                     StepFlags flags)
 {
     constexpr unsigned ALL = 0xffffffffu;
     const unsigned ax = sub & 3u;
@@ -1219,9 +1269,9 @@ __device__ __forceinline__ void integrate_components(const DevParams &P, const D
     }
     const unsigned c = ((unsigned)cz * P.num[1]) * P.num[0] + (unsigned)cy * P.num[0] + (unsigned)cell;
     S.cell_new[k] = c;
-    if (c != S.cell_of[k]) *resort_flag = 1;
+    if (c != S.cell_of[k]) *flags.resort = flags.value;
     const double lim = 0.45 * P.skin;
-    if (drift * drift + dy * dy + dz * dz > lim * lim) *nl_flag = 1;
+    if (drift * drift + dy * dy + dz * dz > lim * lim) *flags.nl = flags.value;
 }
 
 // Copies sorted particle k's x / vel / angvel (and their FP32 copies) into
@@ -1265,12 +1315,11 @@ __device__ __forceinline__ double warp_chunk_tree_sum(const double *in, unsigned
     return v[0];
 }
 
-// The end of a step whose particles k_contacts_integrate advanced, by one
-// warp once every chunk partial is written: the partials added in chunk
-// order (the reference's serial loop, integration.cuh:67-68, 376-378;
-// every lane forms the same sum), then in lane 0 the wall update, the loop
-// counters and the next step's flags.
-__device__ __forceinline__ void finish_step(const DevParams &P, const DevState &S)
+// The walls and the loop counters after a step, by one warp once every chunk
+// partial is written: the partials added in chunk order (the reference's serial
+// loop, integration.cuh:67-68, 376-378; every lane forms the same sum), then in
+// lane 0 the wall update and the clock.  A step with a device error leaves them.
+__device__ __forceinline__ void advance_walls(const DevParams &P, const DevState &S)
 {
     const unsigned lane = threadIdx.x & 31u;
     DevCtl *ctl = S.ctl;
@@ -1289,16 +1338,7 @@ __device__ __forceinline__ void finish_step(const DevParams &P, const DevState &
             v = vn;
         }
     }
-    if (lane != 0) return;
-    ctl->ticket = 0;
-    // the flags the integration raised in the contact launch
-    if (__ldcg(&ctl->resort_next)) ctl->resort = 1;
-    // lists rebuilt at the start of this step are current unless a particle
-    // has since left its skin
-    ctl->nl_rebuild = __ldcg(&ctl->nl_next);
-    ctl->resort_next = 0;
-    ctl->nl_next = 0;
-    if (*(volatile int *)&ctl->err) return;
+    if (lane != 0 || *(volatile int *)&ctl->err) return;
     const long long iter = ctl->iter;
     const double t_current = ctl->t_current;
     walls_integrate(P, S, wforce, iter, t_current);
@@ -1307,35 +1347,73 @@ __device__ __forceinline__ void finish_step(const DevParams &P, const DevState &
     ctl->iter = iter + 1;
 }
 
+// The end of a step whose particles k_contacts_integrate advanced, by one warp
+// once every chunk partial is written: the next step's flags, then the walls
+// and the clock.
+__device__ __forceinline__ void finish_step(const DevParams &P, const DevState &S)
+{
+    DevCtl *ctl = S.ctl;
+    if ((threadIdx.x & 31u) == 0) {
+        ctl->ticket = 0;
+        // the flags the integration raised in the contact launch
+        if (__ldcg(&ctl->resort_next)) ctl->resort = 1;
+        // lists rebuilt at the start of this step are current unless a particle
+        // has since left its skin
+        ctl->nl_rebuild = __ldcg(&ctl->nl_next);
+        ctl->resort_next = 0;
+        ctl->nl_next = 0;
+    }
+    advance_walls(P, S);
+}
+
 // Contacts, forces and integration of the particles k0 .. k0 + pw - 1 by one
-// warp, into the other buffer of the x / vel / angvel pair.  Returns false in
-// the lanes that own a particle whose contact search raised an error, and in
-// those that own none.
-template <int PREC, int MODEL>
+// warp, into the other buffer of the x / vel / angvel pair.  clock() gives the
+// loop state once before_walls() has run.  Returns false in the lanes that own
+// a particle whose contact search raised an error, and in those that own none.
+template <int PREC, int MODEL, bool BONDS, class Clock, class Before = WallsReady>
 __device__ __forceinline__ bool contacts_integrate_warp(const DevParams &P, const DevState &S, unsigned k0,
-                                                        unsigned pw, const WarpScratch &W,
-                                                        const StepClock &clk, int *resort_flag, int *nl_flag)
+                                                        unsigned pw, const WarpScratch &W, Clock &&clock,
+                                                        StepFlags flags, Before &&before_walls = Before())
 {
     const unsigned lane = threadIdx.x & 31u;
     ContactOut c;
     c.F = c.T = mk3(0.0, 0.0, 0.0);
-    const bool got = contact_warp<PREC, MODEL>(P, S, k0, pw, W, c);
-    if (got) contact_writeback(P, S, k0 + lane, c);
+    const bool got = contact_warp<PREC, MODEL>(P, S, k0, pw, W, c, before_walls);
+    if (got) {
+        if (BONDS) (void)add_bonds(S, S.orig_of[k0 + lane], c.F, c.T);
+        contact_writeback(P, S, k0 + lane, c);
+    }
+    const StepClock clk = clock();
     if (pw <= 8u) {
         const unsigned ip = lane & (pw - 1u);
         integrate_components(P, S, k0 + ip, ip, lane / pw, pw, __shfl_sync(0xffffffffu, (int)got, ip), c.F, c.T,
-                             clk, resort_flag, nl_flag);
+                             clk, flags);
     } else if (got) {
         integrate_particle(P, S, k0 + lane, make_double4(c.F.x, c.F.y, c.F.z, 0.0f),
                            make_double4(c.T.x, c.T.y, c.T.z, 0.0f), clk, S.x_nx, S.vel_nx, S.angvel_nx,
-                           S.vel_f_nx, S.angvel_f_nx, resort_flag, nl_flag);
+                           S.vel_f_nx, S.angvel_f_nx, flags);
     }
     return got;
 }
 
+// The loop state as DevCtl holds it (L2: another block may have advanced it in
+// this launch).
+__device__ __forceinline__ StepClock read_clock(const DevCtl *ctl)
+{
+    StepClock clk;
+    clk.iter = __ldcg(&ctl->iter);
+    clk.t_current = __ldcg(&ctl->t_current);
+    clk.velocity_state = __ldcg(&ctl->velocity_state);
+    clk.tau_eff_x = __ldcg(&ctl->tau_eff_x);
+    return clk;
+}
+
 // The contact stage and the particle integration of one DEM step in one
-// launch, for dry boxes without bonds, fluid or a shear-stress wall (their
-// forces would have to join before the integration).  A warp runs the contact
+// launch, for runs without fluid or a shear-stress wall (their forces would
+// have to join before the integration).  Bond forces depend on the state before
+// the step alone: k_bonds has run, and the owners add them (1e6 spheres with
+// 2.3e6 bonds, us per step: 426 with the gather and the integration in launches
+// of their own, 396 so).  A warp runs the contact
 // search and forces of its pw particles, the owners write them back and
 // integrate into the other buffer of the x / vel / angvel ping-pong pair
 // (S.x_nx, ...).  Every partner is read from the current buffer, which no
@@ -1345,7 +1423,7 @@ __device__ __forceinline__ bool contacts_integrate_warp(const DevParams &P, cons
 // update and the loop counters follow in k_walls_step.  After a device error
 // (raised by an earlier step, or by the particle's contact search) the
 // particle's state is carried to the other buffer unchanged.
-template <int PREC, int MODEL>
+template <int PREC, int MODEL, bool BONDS>
 __global__ void __launch_bounds__(SPHB_CONTACT_B, SPHB_CONTACT_MINB)
 k_contacts_integrate(DevParams P, DevState S, unsigned pw)
 {
@@ -1361,12 +1439,114 @@ k_contacts_integrate(DevParams P, DevState S, unsigned pw)
         return;
     }
     const WarpScratch W = contact_warp_scratch<PREC, MODEL>(contact_smem, warp, P.nc);
-    StepClock clk;
-    clk.iter = ctl->iter;
-    clk.t_current = ctl->t_current;
-    clk.velocity_state = ctl->velocity_state;
-    clk.tau_eff_x = ctl->tau_eff_x;
-    if (!contacts_integrate_warp<PREC, MODEL>(P, S, k0, pw, W, clk, &ctl->resort_next, &ctl->nl_next) && own)
+    if (!contacts_integrate_warp<PREC, MODEL, BONDS>(P, S, k0, pw, W, [&] { return read_clock(ctl); }, StepFlags{&ctl->resort_next, &ctl->nl_next, 1}) && own)
+        carry_particle(S, k);
+}
+
+// Bounded wait of one warp until *p == want (acquire): false after ~2^24 polls
+// (DERR_TIMEOUT), or when another block has timed out.
+__device__ __forceinline__ bool wait_equal(const unsigned *p, unsigned want, DevCtl *ctl)
+{
+    unsigned spins = 0;
+    for (;;) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+        if (v == want) return true;
+        if (++spins > (1u << 24)) {
+            raise_err(ctl, DERR_TIMEOUT, -1);
+            return false;
+        }
+        if ((spins & 255u) == 0u && *(volatile int *)&ctl->err == DERR_TIMEOUT) return false;
+    }
+}
+
+// A whole DEM step in one cooperative launch, for systems that fit one wave
+// (dry, no bonds, no shear-stress wall): what k_resort, k_contacts_integrate
+// and k_walls_step do in three.  The step is a few tens of microseconds or
+// less, so each launch costs a tenth of it or more, and so does the serial sum
+// of the wall partials (391 dependent FP64 additions for 100,000 spheres).
+//
+//   * Re-sort and list rebuild when the step before asked for them, with grid
+//     barriers; otherwise nothing waits here.
+//   * The walls of the step before (`pending`) are moved while this step's
+//     contacts are evaluated: the first warps of the blocks form the chunk sums
+//     of its wall forces, block 0 adds them in order, moves the walls, advances
+//     the clock and publishes (DevCtl::ready); the others wait for it only
+//     before they look at the walls.  k_step_end does it for the last step.
+//   * What this step raises for the next goes to the slot of the other view,
+//     stamped with that step's number, so nothing is cleared while another
+//     block may still read it.
+//
+// The wall forces per particle have two buffers, like x, vel and angvel.
+// Block 0 owns no particles; blocks 1.. take 4 pw each.
+// Measured (us per step, B200, three launches / this): 400 spheres 18.0 / 14.1,
+// 10,000 without contacts 16.1 / 13.9, 20,011 viscous 33.0 / 27.9, 100,000 in
+// shear 56.7 / 53.1 mixed and 72.1 / 63.1 faithful FP64.
+template <int PREC, int MODEL>
+__global__ void __launch_bounds__(SPHB_CONTACT_B, SPHB_CONTACT_MINB)
+k_step(DevParams P, DevState S, PermScratch W, unsigned pw, int view, int pending)
+{
+    extern __shared__ __align__(16) unsigned char contact_smem[];
+    constexpr unsigned ALL = 0xffffffffu;
+    const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    DevCtl *ctl = S.ctl;
+    const unsigned stamp = __ldcg(&ctl->stamp[view]);
+    const bool err = __shfl_sync(ALL, *(volatile int *)&ctl->err, 0) != 0;
+    const bool resort = pending ? __ldcg(&ctl->resort_at[view]) == (int)stamp : __ldcg(&ctl->resort) != 0;
+    const bool nl = resort || (pending ? __ldcg(&ctl->nl_at[view]) == (int)stamp : __ldcg(&ctl->nl_rebuild) != 0);
+    const unsigned nb = gridDim.x - 1u;
+    const unsigned nchunks = P.nw > 0 ? P.nblocks256 : 0u;
+    // chunk sums of the pending step's wall forces
+    if (pending && warp == 0 && blockIdx.x > 0 && blockIdx.x <= nchunks) {
+        for (unsigned j = blockIdx.x - 1u; j < nchunks; j += nb) {
+            const double part = warp_chunk_tree_sum(S.walls_force_prev, P.np, j);
+            if (lane == 0) S.partials[j] = part;
+        }
+        if (lane == 0) {
+            __threadfence();
+            atomicAdd(&ctl->ticket, 1u);
+        }
+    }
+    if (resort && !err) {
+        auto bar = [&]() { return grid_barrier(ctl, gridDim.x, (P.inject & kInjectResort) != 0); };
+        if (!resort_group(P, S, W, gridDim.x, blockIdx.x, bar, true) || !bar()) return;
+    }
+    if (blockIdx.x == 0) {
+        if (warp != 0) return;
+        if (pending) {
+            const unsigned summing = min(nb, nchunks);
+            if (!__all_sync(ALL, wait_equal(&ctl->ticket, summing, ctl))) return;
+            advance_walls(P, S);
+        }
+        if (lane == 0) {
+            ctl->ticket = 0;
+            if (resort && !err) ctl->resorts += 1;
+            if (nl && !err) ctl->nl_builds += 1;
+            ctl->stamp[view ^ 1] = stamp + 1u;
+            asm volatile("st.release.gpu.global.u32 [%0], %1;" :: "l"(&ctl->ready), "r"(stamp) : "memory");
+        }
+        return;
+    }
+    const unsigned k0 = ((blockIdx.x - 1u) * (blockDim.x >> 5) + warp) * pw, k = k0 + lane;
+    if (k0 >= P.np) return;   // whole warps
+    const bool own = lane < pw && k < P.np;
+    if (err) {
+        if (own) carry_particle(S, k);
+        return;
+    }
+    if (nl) {
+        if (own) nl_build_particle(P, S, k);
+        __syncwarp();   // the warp's lanes read the lists
+    }
+    const WarpScratch ws = contact_warp_scratch<PREC, MODEL>(contact_smem, warp, P.nc);
+    auto walls = [&] {
+        if (pending) (void)wait_equal(&ctl->ready, stamp, ctl);
+        __syncwarp();
+    };
+    if (!contacts_integrate_warp<PREC, MODEL, false>(P, S, k0, pw, ws, [&] { return read_clock(ctl); },
+                                              StepFlags{&ctl->resort_at[view ^ 1], &ctl->nl_at[view ^ 1],
+                                                        (int)(stamp + 1u)},
+                                              walls) && own)
         carry_particle(S, k);
 }
 

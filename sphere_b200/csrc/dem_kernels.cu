@@ -26,16 +26,19 @@ __global__ void k_occ_from_rows(DevParams P, DevState S)
 // bond state; forces are added per particle in bond order (k_bond_gather)
 // instead of the reference's unsynchronised `+=`.
 // ---------------------------------------------------------------------
+//
+// S.bond_ft holds 6 doubles per bond: the force on its first particle and the
+// torque on its second (zero for a broken bond).
 template <int PREC>
-__global__ void k_bonds(DevParams P, DevState S, double4 *bond_f, double4 *bond_t)
+__global__ void k_bonds(DevParams P, DevState S)
 {
     unsigned idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (S.ctl->err || idx >= P.nb0) return;
     const double dt = P.dt;
     uint2 bond = S.bonds[idx];
-    bond_f[idx] = make_double4(0.0, 0.0, 0.0, 0.0);
-    bond_t[idx] = make_double4(0.0, 0.0, 0.0, -1.0);  // w < 0: no contribution
-    if (!(bond.x < P.np)) return;
+    double2 *ft = S.bond_ft + 3 * (size_t)idx;
+    auto none = [&] { ft[0] = ft[1] = ft[2] = make_double2(0.0, 0.0); };
+    if (!(bond.x < P.np)) { none(); return; }
     if (bond.y >= P.np) { raise_err(S.ctl, DERR_BOND, (int)idx); return; }
     double4 d0 = S.bonds_delta[idx], w0 = S.bonds_omega[idx];
     V3 delta0_t = xyz(d0);
@@ -80,41 +83,27 @@ __global__ void k_bonds(DevParams P, DevState S, double4 *bond_f, double4 *bond_
     double tau_max = vlen<PREC>(f_t) / A + vlen<PREC>(t_n) * R_bar / J;
     if (sigma_max >= P.sigma_b || tau_max >= P.tau_b) {
         S.bonds[idx].x = P.nb0;  // cohesion.cuh:205
+        none();
         return;
     }
     S.bonds_delta[idx] = make_double4(delta_t.x, delta_t.y, delta_t.z, delta_n);
     S.bonds_omega[idx] = make_double4(omega_t.x, omega_t.y, omega_t.z, omega_n);
-    bond_f[idx] = make_double4(f.x, f.y, f.z, 0.0);
-    bond_t[idx] = make_double4(t_j.x, t_j.y, t_j.z, 1.0);
+    ft[0] = make_double2(f.x, f.y);
+    ft[1] = make_double2(f.z, t_j.x);
+    ft[2] = make_double2(t_j.y, t_j.z);
 }
 
-// Adds each particle's bond forces in increasing bond order.  bond_list
-// entries are (bond index << 1) | (1 if the particle is bond.y).
-__global__ void k_bond_gather(DevParams P, DevState S, const double4 *bond_f,
-                              const double4 *bond_t)
+// Adds each particle's bond forces (steps whose contacts do not: with fluid or
+// a shear-stress wall).
+__global__ void k_bond_gather(DevParams P, DevState S)
 {
     unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
     if (S.ctl->err || k >= P.np) return;
-    unsigned o = S.orig_of[k];
-    unsigned b0 = S.bond_ptr[o], b1 = S.bond_ptr[o + 1];
-    if (b0 == b1) return;
     double4 f = S.force[k], tq = S.torque[k];
-    for (unsigned j = b0; j < b1; ++j) {
-        unsigned e = S.bond_list[j];
-        unsigned b = e >> 1;
-        double4 bt = bond_t[b];
-        if (bt.w < 0.0) continue;
-        double4 bf = bond_f[b];
-        if ((e & 1) == 0) {
-            f.x += bf.x; f.y += bf.y; f.z += bf.z; f.w += 0.0;
-            tq.x -= bt.x; tq.y -= bt.y; tq.z -= bt.z; tq.w -= 0.0;
-        } else {
-            f.x -= bf.x; f.y -= bf.y; f.z -= bf.z; f.w -= 0.0;
-            tq.x += bt.x; tq.y += bt.y; tq.z += bt.z; tq.w += 0.0;
-        }
-    }
-    S.force[k] = f;
-    S.torque[k] = tq;
+    V3 F = xyz(f), T = xyz(tq);
+    if (!add_bonds(S, S.orig_of[k], F, T)) return;
+    S.force[k] = make_double4(F.x, F.y, F.z, f.w);
+    S.torque[k] = make_double4(T.x, T.y, T.z, tq.w);
 }
 
 // findShearStressOnFixedMovingParticles, src/integration.cuh:457-484
@@ -205,7 +194,7 @@ __global__ void __launch_bounds__(256, SPHB_INTEGRATE_MINB) k_integrate(DevParam
     clk.tau_eff_x = ctl->tau_eff_x;
     if (ok && k < P.np)
         integrate_particle(P, S, k, S.force[k], S.torque[k], clk, S.x, S.vel, S.angvel, S.vel_f,
-                           S.angvel_f, &ctl->resort, &ctl->nl_rebuild);
+                           S.angvel_f, StepFlags{&ctl->resort, &ctl->nl_rebuild, 1});
     if (P.nw > 0 && P.np > 0) {
         double s = chunk_tree_sum(S.walls_force_pp, P.np, blockIdx.x, cache);
         if (threadIdx.x == 0) S.partials[blockIdx.x] = s;
@@ -259,6 +248,38 @@ __global__ void __launch_bounds__(32 * SPHB_WALLS_WARPS) k_walls_step(DevParams 
     if (!__shfl_sync(0xffffffffu, last, 0)) return;
     __threadfence();
     finish_step(P, S);
+}
+
+// After the last of a run of k_step launches (S and `view` are the view it
+// integrated into): its walls and clock, and the flags of the next step where
+// the other step paths and the host keep them.
+__global__ void __launch_bounds__(32 * SPHB_WALLS_WARPS) k_step_end(DevParams P, DevState S, int view)
+{
+    DevCtl *ctl = S.ctl;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const unsigned nchunks = P.np > 0 ? P.nblocks256 : 1;
+    if (j >= nchunks) return;   // whole warps
+    if (P.nw > 0 && P.np > 0) {
+        const double part = warp_chunk_tree_sum(S.walls_force_prev, P.np, j);
+        if (lane == 0) S.partials[j] = part;
+    }
+    int last = 0;
+    if (lane == 0) {
+        __threadfence();
+        last = atomicAdd(&ctl->ticket, 1u) == nchunks - 1;
+    }
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __threadfence();
+    if (lane == 0) {
+        ctl->ticket = 0;
+        const int stamp = (int)__ldcg(&ctl->stamp[view]);
+        ctl->resort = __ldcg(&ctl->resort_at[view]) == stamp;
+        ctl->nl_rebuild = __ldcg(&ctl->nl_at[view]) == stamp;
+        // numbers only grow, whatever path steps in between
+        ctl->stamp[0] = ctl->stamp[1] = (unsigned)stamp + 1u;
+    }
+    advance_walls(P, S);
 }
 
 // Cell hash of the current positions (first step, after sph_set).
@@ -354,14 +375,18 @@ cudaError_t launch_contacts(const DevParams &P, const DevState &S, int prec, cud
                      : launch_contact_kernel<1, 1>(k_contacts<1, 1>, P, S, st);
 }
 
+template <int PREC, int MODEL>
+static cudaError_t launch_ci(const DevParams &P, const DevState &S, cudaStream_t st)
+{
+    return P.nb0 ? launch_contact_kernel<PREC, MODEL>(k_contacts_integrate<PREC, MODEL, true>, P, S, st)
+                 : launch_contact_kernel<PREC, MODEL>(k_contacts_integrate<PREC, MODEL, false>, P, S, st);
+}
+
 cudaError_t launch_contacts_integrate(const DevParams &P, const DevState &S, int prec,
                                       cudaStream_t st)
 {
-    if (P.contactmodel == 2)
-        return prec == 0 ? launch_contact_kernel<0, 2>(k_contacts_integrate<0, 2>, P, S, st)
-                         : launch_contact_kernel<1, 2>(k_contacts_integrate<1, 2>, P, S, st);
-    return prec == 0 ? launch_contact_kernel<0, 1>(k_contacts_integrate<0, 1>, P, S, st)
-                     : launch_contact_kernel<1, 1>(k_contacts_integrate<1, 1>, P, S, st);
+    if (P.contactmodel == 2) return prec == 0 ? launch_ci<0, 2>(P, S, st) : launch_ci<1, 2>(P, S, st);
+    return prec == 0 ? launch_ci<0, 1>(P, S, st) : launch_ci<1, 1>(P, S, st);
 }
 
 cudaError_t launch_walls_step(const DevParams &P, const DevState &S, cudaStream_t st)
@@ -371,13 +396,67 @@ cudaError_t launch_walls_step(const DevParams &P, const DevState &S, cudaStream_
     return cudaGetLastError();
 }
 
-cudaError_t launch_bonds(const DevParams &P, const DevState &S, int prec, double4 *bf,
-                         double4 *bt, cudaStream_t st)
+cudaError_t launch_step_end(const DevParams &P, const DevState &S, int view, cudaStream_t st)
+{
+    const unsigned chunks = P.np > 0 ? P.nblocks256 : 1;
+    k_step_end<<<blocks_for(chunks, SPHB_WALLS_WARPS), 32 * SPHB_WALLS_WARPS, 0, st>>>(P, S, view);
+    return cudaGetLastError();
+}
+
+const void *step_kernel_fp64(int prec, int model)
+{
+    if (model == 2) return prec == 0 ? (const void *)k_step<0, 2> : (const void *)k_step<1, 2>;
+    return prec == 0 ? (const void *)k_step<0, 1> : (const void *)k_step<1, 1>;
+}
+size_t step_smem_fp64(int model, unsigned nc)
+{
+    return (SPHB_CONTACT_B / 32) * (model == 2 ? contact_warp_bytes<0, 2>(nc) : contact_warp_bytes<0, 1>(nc));
+}
+
+StepShape step_shape(int prec, int model, unsigned np, unsigned nc)
+{
+    StepShape sh;
+    sh.fn = prec == 2 ? step_kernel_mixed(model) : step_kernel_fp64(prec, model);
+    sh.smem = prec == 2 ? step_smem_mixed(model, nc) : step_smem_fp64(model, nc);
+    int dev = 0, sms = 0, fit = 0;
+    if (np == 0 || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, sh.fn, SPHB_CONTACT_B, sh.smem) != cudaSuccess) {
+        cudaGetLastError();
+        return StepShape();
+    }
+    constexpr unsigned warps = SPHB_CONTACT_B / 32;
+    const unsigned blocks = (unsigned)(sms * fit);
+    if (blocks < 2) return StepShape();
+    sh.pw = contact_pw(np, (blocks - 1u) * warps);
+    const unsigned need = blocks_for(np, warps * sh.pw);
+    sh.grid = need + 1u <= blocks ? need + 1u : 0u;
+    return sh;
+}
+
+void step_set_pw(StepShape &sh, unsigned np, unsigned pw)
+{
+    sh.pw = pw;
+    sh.grid = blocks_for(np, SPHB_CONTACT_B / 32 * pw) + 1u;
+}
+
+cudaError_t launch_step(const StepShape &sh, const DevParams &P, const DevState &S, unsigned char *scratch,
+                        int view, int pending, cudaStream_t st)
+{
+    PermScratch W = make_perm_scratch(scratch, P.np);
+    DevParams Pc = P;
+    DevState Sc = S;
+    unsigned pw = sh.pw;
+    void *args[] = {(void *)&Pc, (void *)&Sc, (void *)&W, (void *)&pw, (void *)&view, (void *)&pending};
+    return cudaLaunchCooperativeKernel(sh.fn, dim3(sh.grid), dim3(SPHB_CONTACT_B), args, sh.smem, st);
+}
+
+cudaError_t launch_bonds(const DevParams &P, const DevState &S, int prec, int gather, cudaStream_t st)
 {
     if (P.nb0 == 0) return cudaSuccess;
-    if (prec == 0) k_bonds<0><<<blocks_for(P.nb0, 256), 256, 0, st>>>(P, S, bf, bt);
-    else k_bonds<1><<<blocks_for(P.nb0, 256), 256, 0, st>>>(P, S, bf, bt);
-    k_bond_gather<<<blocks_for(P.np, 256), 256, 0, st>>>(P, S, bf, bt);
+    if (prec == 0) k_bonds<0><<<blocks_for(P.nb0, 256), 256, 0, st>>>(P, S);
+    else k_bonds<1><<<blocks_for(P.nb0, 256), 256, 0, st>>>(P, S);
+    if (gather) k_bond_gather<<<blocks_for(P.np, 256), 256, 0, st>>>(P, S);
     return cudaGetLastError();
 }
 

@@ -30,8 +30,27 @@ cudaError_t launch_contacts_integrate_mixed(const DevParams &P, const DevState &
 // wall reduction, wall update, loop counters and the next step's flags after
 // launch_contacts_integrate
 cudaError_t launch_walls_step(const DevParams &P, const DevState &S, cudaStream_t st);
-cudaError_t launch_bonds(const DevParams &P, const DevState &S, int prec, double4 *bond_f,
-                         double4 *bond_t, cudaStream_t st);
+// One launch per step (k_step) for dry systems that fit one wave: the kernel
+// of a precision and contact model, its launch shape (grid 0: it does not fit),
+// the launch, and the launch that completes a run of steps.  `view` is the
+// state view S shows; pending: the step before was one of these and its walls
+// are still to be moved.
+struct StepShape {
+    const void *fn = nullptr;
+    size_t smem = 0;
+    unsigned pw = 0, grid = 0;
+};
+const void *step_kernel_mixed(int model);
+size_t step_smem_mixed(int model, unsigned nc);
+// the same with pw particles per warp (at least as many: it still fits)
+void step_set_pw(StepShape &sh, unsigned np, unsigned pw);
+StepShape step_shape(int prec, int model, unsigned np, unsigned nc);
+cudaError_t launch_step(const StepShape &sh, const DevParams &P, const DevState &S, unsigned char *scratch,
+                        int view, int pending, cudaStream_t st);
+cudaError_t launch_step_end(const DevParams &P, const DevState &S, int view, cudaStream_t st);
+// bond state and forces; gather = 1 also adds them to S.force / S.torque
+// (k_contacts_integrate adds them itself)
+cudaError_t launch_bonds(const DevParams &P, const DevState &S, int prec, int gather, cudaStream_t st);
 // shear-stress reduction (wmode 3), then one kernel: integration, wall
 // reduction + wall integration, loop counters
 cudaError_t launch_integrate(const DevParams &P, const DevState &S, cudaStream_t st);

@@ -31,10 +31,25 @@ cudaError_t launch_contacts_mixed(const DevParams &P, const DevState &S, cudaStr
                                : launch_contact_kernel<2, 1>(k_contacts<2, 1>, P, S, st);
 }
 
+template <int MODEL>
+static cudaError_t launch_ci(const DevParams &P, const DevState &S, cudaStream_t st)
+{
+    return P.nb0 ? launch_contact_kernel<2, MODEL>(k_contacts_integrate<2, MODEL, true>, P, S, st)
+                 : launch_contact_kernel<2, MODEL>(k_contacts_integrate<2, MODEL, false>, P, S, st);
+}
+
 cudaError_t launch_contacts_integrate_mixed(const DevParams &P, const DevState &S, cudaStream_t st)
 {
-    return P.contactmodel == 2 ? launch_contact_kernel<2, 2>(k_contacts_integrate<2, 2>, P, S, st)
-                               : launch_contact_kernel<2, 1>(k_contacts_integrate<2, 1>, P, S, st);
+    return P.contactmodel == 2 ? launch_ci<2>(P, S, st) : launch_ci<1>(P, S, st);
+}
+
+const void *step_kernel_mixed(int model)
+{
+    return model == 2 ? (const void *)k_step<2, 2> : (const void *)k_step<2, 1>;
+}
+size_t step_smem_mixed(int model, unsigned nc)
+{
+    return (SPHB_CONTACT_B / 32) * (model == 2 ? contact_warp_bytes<2, 2>(nc) : contact_warp_bytes<2, 1>(nc));
 }
 
 int Engine::mixed_init() { return ST_OK; }

@@ -50,6 +50,7 @@ struct DevState {
     double4 *wnx, *wmvfd;
     double *wacc;
     double *walls_force_pp;   // nw * np, ORIGINAL order (reduced like the reference)
+    double *walls_force_prev; // those of the step before (the other view's buffer)
     double *tau_pp;           // np, ORIGINAL order
     double *partials;         // nblocks256
     double *tau_partials;     // nblocks256
@@ -59,6 +60,7 @@ struct DevState {
     double4 *bonds_delta, *bonds_omega;
     // per-particle bond lists (CSR over original index) for gather accumulation
     uint32_t *bond_ptr, *bond_list;
+    double2 *bond_ft;      // force and torque of each bond (3 per bond), null without bonds
 
     // sort scratch
     uint32_t *count, *fill, *vals, *block_sums;

@@ -73,6 +73,13 @@ struct DevCtl {
     // nl_rebuild once that launch has finished
     int resort_next;
     int nl_next;
+    // k_step (one launch per step): the number of the step that runs on each
+    // view, what the step before asked for (by that number, in the slot of the
+    // step's view), and the last step whose predecessor's walls are moved
+    unsigned stamp[2];
+    int resort_at[2];
+    int nl_at[2];
+    unsigned ready;
 };
 
 struct V3 {

@@ -67,6 +67,7 @@ Engine::~Engine()
     darcy_free();
     ns_free();
     persist_free();
+    delete step_one;
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     for (ShortGraph &g : short_graph)
         if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -164,11 +165,14 @@ int Engine::allocate_and_upload()
         S.delta_t_f = dalloc<float4>(slots);
     }
     // the other buffer of the x / vel / angvel pair for the fused step paths
-    if (fused_eligible() && step_kernel != 1 && step_kernel != 3) {
+    if ((fused_eligible() && step_kernel != 1 && step_kernel != 3) || bonded_fused()) {
         S.x_nx = dalloc<double4>(n); S.vel_nx = dalloc<double4>(n); S.angvel_nx = dalloc<double4>(n);
         if (precision == SPH_PREC_MIXED) {
             S.vel_f_nx = dalloc<float4>(n);
             S.angvel_f_nx = dalloc<float4>(n);
+        }
+        if (step_kernel != 2 && h.nb0 == 0) {
+            step_one = new StepShape(step_shape(precision, (int)h.contactmodel, h.np, capacity));
         }
         if (!S.x_nx || !S.vel_nx || !S.angvel_nx) return fail(ST_CUDA, "device allocation failed");
     }
@@ -178,7 +182,9 @@ int Engine::allocate_and_upload()
     S.nl_count = dalloc<uint32_t>(n);
     S.x_ref = dalloc<float4>(n);
     S.wnx = dalloc<double4>(6); S.wmvfd = dalloc<double4>(6); S.wacc = dalloc<double>(6);
-    S.walls_force_pp = dalloc<double>(n * (h.nw ? h.nw : 1));
+    const size_t wall_values = n * (h.nw ? h.nw : 1);
+    S.walls_force_pp = dalloc<double>(step_one ? 2 * wall_values : wall_values);
+    if (step_one && S.walls_force_pp) S.walls_force_prev = S.walls_force_pp + wall_values;
     S.tau_pp = dalloc<double>(n);
     S.partials = dalloc<double>(P.nblocks256 + 1);
     S.tau_partials = dalloc<double>(P.nblocks256 + 1);
@@ -190,8 +196,7 @@ int Engine::allocate_and_upload()
     S.block_sums = dalloc<uint32_t>(4096);
     S.perm_scratch = dalloc<unsigned char>(resort_scratch_bytes(n));
     S.ctl = dalloc<DevCtl>(1);
-    bond_f = dalloc<double4>(h.nb0);
-    bond_t = dalloc<double4>(h.nb0);
+    if (h.nb0) S.bond_ft = dalloc<double2>(3 * (size_t)h.nb0);
     tmp = dalloc<unsigned char>(std::max<size_t>(slots * 32, n * 32) + 64);
     if (alloc_failed) return fail(ST_CUDA, "device allocation failed");
 
@@ -323,7 +328,7 @@ cudaError_t Engine::enqueue_stage(int stage)
         if (precision == SPH_PREC_MIXED)
             return launch_contacts_mixed(P, S, stream, step_kernel == 3);
         return launch_contacts(P, S, prec, stream, step_kernel == 3);
-    case 2: return launch_bonds(P, S, prec, bond_f, bond_t, stream);
+    case 2: return launch_bonds(P, S, prec, !fused, stream);
     case 3: return enqueue_fluid();
     case 4:
         if (fused) {
@@ -337,10 +342,34 @@ cudaError_t Engine::enqueue_stage(int stage)
     }
 }
 
+// Enqueues n steps of the current path: one launch each where k_step covers
+// them, and the launch that completes them.
+cudaError_t Engine::enqueue_steps(uint64_t n)
+{
+    cudaError_t e = cudaSuccess;
+    if (!(fused && step_one && step_one->grid)) {
+        for (uint64_t i = 0; i < n && e == cudaSuccess; ++i) e = enqueue_step();
+        return e;
+    }
+    for (uint64_t i = 0; i < n && e == cudaSuccess; ++i) {
+        e = launch_step(*step_one, P, S, S.perm_scratch, cur_view, i > 0, stream);
+        if (e == cudaSuccess) flip_view();
+    }
+    if (e == cudaSuccess && n > 0) e = launch_step_end(P, S, cur_view, stream);
+    return e;
+}
+
+// The stages of a step in their order: bonds before the contacts that add them.
+const int *Engine::stage_order() const
+{
+    static const int plain[5] = {0, 1, 2, 3, 4}, bonded[5] = {0, 2, 1, 3, 4};
+    return fused && hs.nb0 ? bonded : plain;
+}
+
 cudaError_t Engine::enqueue_step()
 {
-    for (int st = 0; st < 5; ++st) {
-        cudaError_t e = enqueue_stage(st);
+    for (int q = 0; q < 5; ++q) {
+        cudaError_t e = enqueue_stage(stage_order()[q]);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -356,7 +385,7 @@ int Engine::profile(uint64_t n, sph_profile *out)
     for (uint64_t i = 0; i < n && rc == ST_OK; ++i) {
         cudaEventRecord(ev[0], stream);
         for (int st = 0; st < 5; ++st) {
-            cudaError_t e = enqueue_stage(st);
+            cudaError_t e = enqueue_stage(stage_order()[st]);
             if (e != cudaSuccess) { rc = cuda_fail(e, "profile"); break; }
             cudaEventRecord(ev[st + 1], stream);
         }
@@ -365,7 +394,7 @@ int Engine::profile(uint64_t n, sph_profile *out)
         for (int st = 0; st < 5; ++st) {
             float t = 0;
             cudaEventElapsedTime(&t, ev[st], ev[st + 1]);
-            ms[st] += t;
+            ms[stage_order()[st]] += t;
         }
         float t = 0;
         cudaEventElapsedTime(&t, ev[0], ev[5]);
@@ -411,7 +440,7 @@ cudaGraphExec_t Engine::capture_steps(int k)
     const int view0 = cur_view;   // fused steps flip the view while they are captured
     cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
-    for (int i = 0; i < k && e == cudaSuccess; ++i) e = enqueue_step();
+    e = enqueue_steps((uint64_t)k);
     cudaError_t e2 = cudaStreamEndCapture(stream, &g);
     if (e != cudaSuccess || e2 != cudaSuccess || !g) {
         if (g) cudaGraphDestroy(g);
@@ -447,13 +476,13 @@ int Engine::step_stages(uint64_t n)
         int rc = poll_errors("step");
         if (rc) return rc;
     }
-    ensure_graph();
     uint64_t done = 0;
     const uint64_t glen = (uint64_t)graph_len();
-    // a program that steps in short calls of one length replays them too, from
-    // the second such call on (per view: an odd number of fused steps ends on
-    // the other one)
-    if (n >= 4 && n < glen && graph_steps > 1 && !graph_failed) {
+    if (n >= glen) ensure_graph();
+    // a program that steps in calls of one length, up to a few of these graphs,
+    // replays the whole call from the second one on (per view: an odd number of
+    // fused steps ends on the other one)
+    if (n >= 4 && n <= 4 * glen && n != glen && graph_steps > 1 && !graph_failed) {
         ShortGraph &g = short_graph[cur_view];
         const bool seen = g.n == n && g.fused == fused;
         if (!seen && g.exec) {
@@ -477,10 +506,8 @@ int Engine::step_stages(uint64_t n)
         if (e != cudaSuccess) return cuda_fail(e, "graph launch");
         done += glen;
     }
-    for (; done < n; ++done) {
-        cudaError_t e = enqueue_step();
-        if (e != cudaSuccess) return cuda_fail(e, "step");
-    }
+    cudaError_t e = enqueue_steps(n - done);
+    if (e != cudaSuccess) return cuda_fail(e, "step");
     advance_host_clock(n);
     return poll_errors("step");
 }
@@ -915,7 +942,7 @@ static int open_common(std::unique_ptr<Engine> &eng, const sph_opts *opts)
     if (e.step_kernel == 4 && !e.fused_eligible())
         return e.fail(sphb::ST_UNSUPPORTED, "contacts and integration in one launch do not cover "
                                             "bonds, fluid or the shear-stress wall (wmode 3)");
-    e.fused = e.step_kernel == 4;
+    e.fused = e.step_kernel == 4 || e.bonded_fused();
     rc = e.allocate_and_upload();
     if (rc) return rc;
     rc = e.darcy_init();

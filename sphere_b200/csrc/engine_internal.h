@@ -18,6 +18,7 @@ namespace sphb {
 struct DarcyDev;   // Darcy solver state (darcy.cu)
 struct NSDev;      // Navier-Stokes solver state (navierstokes.cu)
 struct MixedDev;   // mixed-precision state (dem_mixed.cu)
+struct StepShape;  // one launch per step (dem_launch.h)
 struct PersistDev; // fused persistent step path (engine_persist.cu)
 
 // FP32 velocity copies of the mixed mode from the FP64 velocities.
@@ -51,7 +52,6 @@ public:
     bool alloc_failed = false;    // a dalloc() returned null
     void *host_pinned = nullptr;
     unsigned char *tmp = nullptr;
-    double4 *bond_f = nullptr, *bond_t = nullptr;
 
     // loop state mirrored on the host (same double additions as the device)
     double host_t = 0.0;
@@ -63,7 +63,7 @@ public:
     int graph_view = -1;          // state view the graph was captured with
     bool graph_fused = false;     // the graph holds fused per-stage steps
     bool graph_failed = false;
-    // graph of one call of n < graph_steps steps, per state view
+    // graph of one call of n steps, per state view
     struct ShortGraph {
         cudaGraphExec_t exec = nullptr;
         uint64_t n = 0;
@@ -107,7 +107,10 @@ public:
     int allocate_and_upload();
     int poll_errors(const char *where);
     cudaError_t enqueue_stage(int stage);
+    const int *stage_order() const;
     cudaError_t enqueue_step();
+    cudaError_t enqueue_steps(uint64_t n);
+    StepShape *step_one = nullptr;   // k_step's launch (null: not this engine)
     cudaError_t enqueue_fluid();
     int profile(uint64_t n, struct sph_profile *out);
     int ensure_graph();
@@ -163,7 +166,9 @@ public:
 
     // fused per-stage step path
     bool fused_eligible() const;
+    bool bonded_fused() const;
     void set_fused(bool on);
+    void set_step_pw(unsigned pw);
     void flip_view();
     int graph_len() const;
 

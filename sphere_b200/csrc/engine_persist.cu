@@ -53,6 +53,12 @@ bool Engine::fused_eligible() const
     return !hs.fluid && hs.nb0 == 0 && !(hs.nw > 0 && hs.wmode[0] == 3) && hs.np > 0;
 }
 
+// Runs with bonds that the automatic choice steps with k_contacts_integrate.
+bool Engine::bonded_fused() const
+{
+    return step_kernel == 0 && hs.nb0 > 0 && !hs.fluid && !(hs.nw > 0 && hs.wmode[0] == 3) && hs.np > 0;
+}
+
 bool Engine::persist_eligible() const
 {
     if (step_kernel != 0 && step_kernel != 2) return false;
@@ -71,6 +77,22 @@ void Engine::set_fused(bool on)
     if (graph_exec) {
         cudaGraphExecDestroy(graph_exec);
         graph_exec = nullptr;
+    }
+}
+
+// Particles per warp of the one-launch step (results do not depend on it);
+// graphs hold the launch, so they go.
+void Engine::set_step_pw(unsigned pw)
+{
+    if (!step_one->grid || step_one->pw == pw) return;
+    step_set_pw(*step_one, hs.np, pw);
+    if (graph_exec) {
+        cudaGraphExecDestroy(graph_exec);
+        graph_exec = nullptr;
+    }
+    for (ShortGraph &g : short_graph) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        g = ShortGraph();
     }
 }
 
@@ -96,6 +118,7 @@ void Engine::make_views()
     std::swap(S_view[1].angvel, S_view[1].angvel_nx);
     std::swap(S_view[1].vel_f, S_view[1].vel_f_nx);
     std::swap(S_view[1].angvel_f, S_view[1].angvel_f_nx);
+    if (S_view[1].walls_force_prev) std::swap(S_view[1].walls_force_pp, S_view[1].walls_force_prev);
 }
 
 int Engine::persist_init()
@@ -192,16 +215,22 @@ int Engine::step_persistent(uint64_t n)
     uint64_t done = 0;
     const uint64_t trial = 8;
     // candidates: every block shape of the persistent kernel, then (unless
-    // the persistent path was requested) the per-stage kernels and the
-    // per-stage kernels with contacts and integration in one launch
-    const int ncand = kNumPersistShapes + (step_kernel == 2 ? 0 : 2);
-    // calls too short to tune on run the fused per-stage kernels (20,011
-    // spheres: 33 us per step against 50 on the untuned persistent shape)
-    if (!D.tuned && step_kernel != 2 && n < trial * (uint64_t)(ncand + 2)) {
+    // the persistent path was requested) the per-stage kernels and one launch
+    // per step, the latter also with fewer lanes per particle: a system without
+    // contacts has no use for them (10,000 spheres falling apart: 13.9 us
+    // per step against 14.4)
+    const unsigned pw_fine = step_one ? step_one->pw : 32u, pw_coarse = std::min(32u, pw_fine * 4u);
+    const bool coarse = step_one && step_one->grid && pw_coarse != pw_fine;
+    const int ncand = kNumPersistShapes + (step_kernel == 2 ? 0 : coarse ? 3 : 2);
+    // steps the trials take: 8 per shape, 1 + 8 + 8 per candidate of the others
+    const uint64_t trials = std::max(trial * (uint64_t)(ncand + 2),
+                                     trial * kNumPersistShapes +
+                                         (2 * trial + 1) * (uint64_t)(ncand - kNumPersistShapes));
+    if (!D.tuned && step_kernel != 2 && n < trials) {
         set_fused(true);
         return step_stages(n);
     }
-    if (!D.tuned && n >= trial * (uint64_t)(ncand + 2)) {
+    if (!D.tuned && n >= trials) {
         cudaEvent_t a, b;
         cudaEventCreate(&a);
         cudaEventCreate(&b);
@@ -214,7 +243,8 @@ int Engine::step_persistent(uint64_t n)
             unsigned g = stages ? 1 : persist_grid(cand);
             if (!g) continue;
             if (stages) {
-                set_fused(cand == kNumPersistShapes + 1);
+                set_fused(cand != kNumPersistShapes);
+                if (step_one) set_step_pw(cand == kNumPersistShapes + 2 ? pw_coarse : pw_fine);
                 if (trial_graph) {
                     cudaGraphExecDestroy(trial_graph);
                     trial_graph = nullptr;
@@ -253,7 +283,8 @@ int Engine::step_persistent(uint64_t n)
         D.tuned = true;
         if (best_cand >= kNumPersistShapes) {
             persist_off = true;
-            set_fused(best_cand == kNumPersistShapes + 1);
+            set_fused(best_cand != kNumPersistShapes);
+            if (step_one) set_step_pw(best_cand == kNumPersistShapes + 2 ? pw_coarse : pw_fine);
             return step_stages(n - done);
         }
         set_fused(false);
@@ -274,9 +305,7 @@ int Engine::step_persistent(uint64_t n)
 cudaError_t Engine::launch_trial_steps(cudaGraphExec_t g, uint64_t n)
 {
     if (g) return cudaGraphLaunch(g, stream);
-    cudaError_t e = cudaSuccess;
-    for (uint64_t i = 0; i < n && e == cudaSuccess; ++i) e = enqueue_step();
-    return e;
+    return enqueue_steps(n);
 }
 
 // After n per-stage trial steps: the host clock and device errors.

@@ -267,7 +267,8 @@ __global__ void __launch_bounds__(NT, MINB) k_persistent(BatchArgs A)
                         if (lane < pw && k < P.np) nl_build_particle(P, S, k);
                         __syncwarp();   // the warp's lanes read the list
                     }
-                    contacts_integrate_warp<PREC, MODEL>(P, S, k0, pw, ws, clk, fr, fn);
+                    contacts_integrate_warp<PREC, MODEL, false>(P, S, k0, pw, ws, [&] { return clk; },
+                                                         StepFlags{fr, fn, 1});
                     __syncwarp();
                 }
             }

@@ -17,6 +17,43 @@
 
 namespace sphb {
 
+// Grid-wide barrier for a cooperative launch, with a bounded wait: after
+// ~2^24 polls (well over a second) it records DERR_TIMEOUT and returns
+// false instead of spinning forever.  With `inject` no block releases it and
+// every block gives up after kInjectPolls polls.
+__device__ __forceinline__ bool grid_barrier(DevCtl *ctl, unsigned nblocks, bool inject)
+{
+    __syncthreads();
+    __shared__ int ok;
+    if (threadIdx.x == 0) {
+        volatile unsigned *gen = &ctl->barrier_gen;
+        unsigned g = *gen;
+        __threadfence();
+        unsigned arrived = atomicAdd(&ctl->barrier_count, 1u);
+        ok = 1;
+        if (arrived == nblocks - 1 && !inject) {
+            ctl->barrier_count = 0;
+            __threadfence();
+            atomicAdd(&ctl->barrier_gen, 1u);
+        } else {
+            unsigned spins = 0;
+            const unsigned limit = inject ? kInjectPolls : (1u << 24);
+            while (inject || *gen == g) {
+                if (++spins > limit) {
+                    raise_err(ctl, DERR_TIMEOUT, -1);
+                    ok = 0;
+                    break;
+                }
+                if (((volatile int *)&ctl->err)[0] == DERR_TIMEOUT) { ok = 0; break; }
+                __nanosleep(64);
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
 // Block-wide exclusive scan of one value per thread (blockDim a multiple of
 // 32, at most 1024).
 __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned &total)

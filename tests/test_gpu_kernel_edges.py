@@ -7,6 +7,7 @@
   and particle counts around their multiples, wide ones (the image plane has no
   height), tall ones (rows repeat), and an eye among the spheres, pixel for pixel
   against the renderer that tests every sphere.
+* One launch per step, with re-sorts inside it, against the oracle.
 * The Darcy iteration keeps one, two or four cells per thread in registers and
   leaves out those that cannot change.
 """
@@ -95,3 +96,22 @@ def test_darcy_cells_per_thread(tmp_path, grid, lid):
             for f in ("darcy_p", "darcy_v", "darcy_phi"):
                 a, b = numpy.ravel(e.get(f)), numpy.ravel(orc.get(f))
                 assert numpy.abs(a - b).max() <= RTOL * max(numpy.abs(b).max(), 1e-300), f
+
+
+# one launch per step: re-sorts inside it, the walls one launch behind, calls of
+# one odd length replayed from a graph on either view
+@pytest.mark.parametrize("n,model", [(400, 2), (5000, 1)])
+def test_one_launch_steps_with_resorts(tmp_path, n, model):
+    from sphere_b200.engine import Engine
+    d = pressed(n, model=model)
+    d.vel = numpy.random.default_rng(7).uniform(-20.0, 20.0, size=(n, 3))   # some sphere changes cell on most steps
+    path = str(tmp_path / "resort.bin")
+    binfile.write_bin(d, path)
+    orc = O.Oracle(path)
+    with Engine(path, step_kernel="stages_fused") as e:
+        for steps in (3, 5, 5, 5, 5, 40):
+            assert orc.step(steps) == 0, orc.error()
+            assert e.step(steps) == 0
+            bad = compare(e, orc)
+            assert not bad, (steps, bad)
+        assert e.info().resorts > 5
