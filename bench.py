@@ -41,14 +41,12 @@ sys.path.insert(0, ROOT)
 
 INTERVAL = 100          # DEM steps per benchmark step
 N_PARTICLES = 100000
-# dram__bytes_read.sum + dram__bytes_write.sum of one k_contacts<2,2> launch
-# on this workload (mixed precision, N = 1e5), from an ncu --set full
-# capture of that kernel: 46.30 MB read + 3.15 MB written (ncu flushes the
-# caches before the launch)
-CONTACTS_TRAFFIC = 46.30e6 + 3.15e6
-# the same for one k_contacts_integrate<2,2> launch (contacts and
-# integration in one launch): 43.62 MB read + 10.41 MB written
-FUSED_TRAFFIC = 43.62e6 + 10.41e6
+# dram__bytes_read.sum + dram__bytes_write.sum of one k_contacts_integrate<2,2>
+# launch (contacts and integration in one launch, which profile() times stage by
+# stage) on this workload (mixed precision, N = 1e5), from an ncu capture of that
+# kernel: 49.62 MB read + 13.57 MB written (ncu flushes the caches before the
+# launch)
+FUSED_TRAFFIC = 49.62e6 + 13.57e6
 SEED = 1
 
 
@@ -276,7 +274,7 @@ def run_gpu(args):
     # partner id 4 + tangential history 24, read and written (56)
     bytes_per_particle = 184.0 + 56.0 * zbar
     kernel_name = "k_contacts (contact search + forces)"
-    traffic = CONTACTS_TRAFFIC if precision == "mixed" else None
+    traffic = None
     if info.step_path == 2:
         # contacts and integration in one launch: the integration's own
         # fields (fixvel 8; angpos, acc0, angacc0, xyzsum read 96; pos, vel,
@@ -289,13 +287,13 @@ def run_gpu(args):
     achieved = contacts_bytes / (prof.contacts_ms * 1e-3) / 1e9
     # launches of this library's kernels in the timed region: per DEM step
     # k_resort (with the list rebuild), k_contacts, k_integrate (+2 for the
-    # shear-stress wall, +2 with bonds) on the per-stage path; k_resort,
-    # k_contacts_integrate and k_walls_step with contacts and integration in
-    # one launch; one k_persistent per call on the persistent path
+    # shear-stress wall, +2 with bonds) on the per-stage path; one k_step, and a
+    # k_step_end per call, with contacts and integration in one launch (systems
+    # of one wave, as this one); one k_persistent per call on the persistent path
     if info.step_path == 1:
         timed_launches = args.steps
     elif info.step_path == 2:
-        timed_launches = 3 * INTERVAL * args.steps
+        timed_launches = (INTERVAL + 1) * args.steps
     else:
         per_step = 3 + (2 if d.nw > 0 and d.wmode[0] == 3 else 0) + (2 if d.nb0 > 0 else 0)
         timed_launches = per_step * INTERVAL * args.steps
@@ -563,7 +561,11 @@ def large_leg(args):
     fp64_rate = n * interval * len(times_fp64) / (float(numpy.sum(times_fp64)) * 1e-3)
     peak, peak_kind = load_peaks()
     step_s = float(numpy.sum(times)) * 1e-3
+    # contacts, bond sums and integration in one launch also move the
+    # integration's own fields (272) and 52 bytes per bond side
     contacts_bpp = 184.0 + 56.0 * zbar
+    if info.step_path == 2:
+        contacts_bpp += 272.0 + 2.0 * 52.0 * nb0 / n
     contacts_gbs = n * contacts_bpp / (prof.contacts_ms * 1e-3) / 1e9
     sort_gbs = n * 228.0 / (sort_ms * 1e-3) / 1e9
     return {
