@@ -68,7 +68,8 @@ typedef struct sph_opts {
                              when its first residual is smaller */
     int graph_steps;      /* DEM steps captured per CUDA graph launch; 0 = automatic */
     const char *output_dir; /* directory for .bin/status/conv outputs; NULL = "output" */
-    int step_kernel;      /* 0 automatic (the fused persistent step where it applies),
+    int step_kernel;      /* 0 automatic (the fastest of the paths below that apply, timed
+                             on the first steps of a long call),
                              1 per-stage kernels, 2 fused persistent step (error where
                              it does not apply: bonds, fluid, wmode 3), 3 per-stage
                              kernels with the contact search reading its partners
@@ -76,7 +77,8 @@ typedef struct sph_opts {
                              (same results; slower on the measured workloads),
                              4 per-stage kernels with the contact search and the
                              particle integration in one launch, integrating into
-                             a second buffer of x / vel / angvel (same results;
+                             a second buffer of x / vel / angvel; the whole step in
+                             one launch where the system fits one wave (same results;
                              error where it does not apply: bonds, fluid, wmode 3) */
     int darcy_exact_stop; /* 1: the Darcy Jacobi loop tests the residual at every
                              iteration and stops at the first that meets the
@@ -167,7 +169,8 @@ typedef struct sph_info {
     uint32_t step_count;
     int64_t resorts;      /* re-sorts performed (steps where a particle changed cell) */
     int32_t step_path;    /* 0 per-stage kernels, 1 fused persistent step, 2 per-stage
-                             kernels with contacts and integration in one launch */
+                             kernels with contacts and integration in one launch (the
+                             whole step in one where the system fits one wave) */
     int32_t step_threads; /* persistent path: threads per block chosen by the autotuner */
     int32_t step_grid;    /* persistent path: blocks of the launch */
     int32_t tuned;        /* 1 once the autotuner has run */
