@@ -115,3 +115,32 @@ def test_one_launch_steps_with_resorts(tmp_path, n, model):
             bad = compare(e, orc)
             assert not bad, (steps, bad)
         assert e.info().resorts > 5
+
+
+# more neighbours than a list holds (48): the particle scans the cells instead
+@pytest.mark.parametrize("model", [1, 2])
+def test_full_neighbour_list(tmp_path, model):
+    from sphere_b200.engine import Engine
+    m, R, r = 60, 0.05, 0.01
+    d = configs.settling_lattice(n=m + 1, seed=9, nx=4, ny=4, nz=4, contactmodel=model)
+    k = numpy.arange(m) + 0.5
+    phi, th = numpy.arccos(1.0 - 2.0 * k / m), numpy.pi * (1.0 + 5.0 ** 0.5) * k
+    shell = numpy.column_stack([numpy.cos(th) * numpy.sin(phi), numpy.sin(th) * numpy.sin(phi), numpy.cos(phi)])
+    d.x = 0.2 + numpy.vstack([numpy.zeros((1, 3)), (R + r - 1e-5) * shell])
+    d.radius = numpy.concatenate([[R], numpy.full(m, r)])
+    d.gamma_n = d.gamma_t = 20.0
+    configs.grid_for(d, L=[0.4, 0.4, 0.4], dx=0.13)
+    path = str(tmp_path / "full.bin")
+    binfile.write_bin(d, path)
+    orc = O.Oracle(path, nc=64)
+    engines = {s: Engine(path, capacity=64, step_kernel=s) for s in ("stages", "stages_fused", "persistent")}
+    for steps in (1, 6):
+        assert orc.step(steps) == 0, orc.error()
+        for s, e in engines.items():
+            assert e.step(steps) == 0
+            bad = compare(e, orc)
+            assert not bad, (s, bad)
+    if model == 2:
+        assert (orc.get("contacts").reshape(m + 1, 64)[0] != m + 1).sum() > 48
+    for e in engines.values():
+        e.close()
