@@ -241,11 +241,13 @@ __global__ void __launch_bounds__(kRtThreads) k_render(const Camera *cam, const 
     auto reaches = [&](float4 b) { return b.x <= bx1 && b.z >= bx0 && b.y <= by1 && b.w >= by0; };
     float tdist = 1e10f, thit = 0.f;
     unsigned hit = 0xffffffffu, hito = 0xffffffffu;   // sorted position and original index
+    // spheres in the list, as the block barrier counts them: the same number in
+    // every thread, while `count` may already be growing with the next turn
+    unsigned staged = 0;
     // the spheres in the list against this thread's pixel
     auto trace = [&]() {
-        const unsigned m = count;
         if (active)
-            for (unsigned q = 0; q < m; ++q) {
+            for (unsigned q = 0; q < staged; ++q) {
                 const float4 x = sx[q];
                 const F3 c = f3(x.x, x.y, x.z);
                 const float R = x.w;
@@ -292,10 +294,11 @@ __global__ void __launch_bounds__(kRtThreads) k_render(const Camera *cam, const 
                 sx[pos] = xr[k];
                 sk[pos] = k;
             }
-            __syncthreads();
-            if (count > kRtList - kRtThreads) {
+            staged += (unsigned)__syncthreads_count(take);
+            if (staged > kRtList - kRtThreads) {
                 trace();
                 __syncthreads();
+                staged = 0u;
                 if (t == 0) count = 0u;
                 __syncthreads();
             }

@@ -71,6 +71,25 @@ def test_render_tiles(n, w, h, scale):
             assert numpy.array_equal(img[:, :, :3], ref[:, :, :3]), (n, w, h, method)
 
 
+# a tile stages spheres 256 at a time and traces them when more than 256 are
+# there: every tile of these images meets hundreds to thousands
+@pytest.mark.parametrize("n,scale", [(257, 12.0), (600, 12.0), (3000, 1.0), (3000, 5.0)])
+def test_render_tiles_with_many_spheres(n, scale):
+    import render_oracle as R
+    from sphere_b200.engine import Engine
+    d = configs.settling_lattice(n=n, seed=104, nx=15, ny=15, nz=15, spacing=0.0195)
+    d.radius = d.radius * scale
+    with Engine(d, precision="faithful") as e:
+        x, vel = e.get("x"), e.get("vel")
+        for w, h in ((16, 16), (33, 33)):
+            val = R.method_values(2, x, vel, e.get("angvel"), e.get("xyzsum"), e.get("angpos"), e.get("p"))
+            ref = R.render(x, vel, d.L, w, h, method=2, val=val, max_val=0.02)
+            assert (ref[:, :, :3] != 255).any()
+            for _ in range(5):
+                img = e.render(method=2, max_val=0.02, width=w, height=h)
+                assert numpy.array_equal(img[:, :, :3], ref[:, :, :3]), (n, w, h)
+
+
 # cells that change: one, two or four per thread of the solver's 148 x 256
 # threads, and a lid of cells that stay as they are
 @pytest.mark.parametrize("grid,lid", [((8, 8, 9), 2), ((33, 35, 32), 0), ((40, 40, 60), 3), ((40, 40, 80), 0)])
