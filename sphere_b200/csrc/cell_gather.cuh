@@ -88,9 +88,12 @@ __device__ __forceinline__ double gather_cells(const DevParams &P, const DevStat
             if (queued >= 32u) {
                 flush(32u);
                 queued -= 32u;
+                // the rest moves to the front: written by the lanes that hold it
+                // alone, before any lane queues behind it
                 const uint32_t e = W.queue[32u + lane];
                 __syncwarp();
-                W.queue[lane] = e;
+                if (lane < queued) W.queue[lane] = e;
+                __syncwarp();
             }
         }
     }

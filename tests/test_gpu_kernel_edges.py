@@ -117,6 +117,66 @@ def test_darcy_cells_per_thread(tmp_path, grid, lid):
                 assert numpy.abs(a - b).max() <= RTOL * max(numpy.abs(b).max(), 1e-300), f
 
 
+def crowded_cells():
+    """Some 200 spheres in reach of each of 4 x 4 x 5 fluid cells."""
+    d = configs.settling_lattice(n=1700, seed=52, nx=12, ny=12, nz=12, spacing=0.0195, steps=40)
+    d.num = numpy.array([4, 4, 5], dtype=numpy.uint32)
+    d.L = numpy.array([0.234, 0.234, 0.29])
+    return d
+
+
+# the porosity kernels queue the spheres of a cell and evaluate them 32 at a time:
+# queues that run over several times.  Bound: about 220 additions of positive
+# terms below the cell's volume, 1.1e-16 each, and the last bits of pow
+def test_darcy_porosity_of_crowded_cells(tmp_path):
+    from sphere_b200.engine import Engine
+    d = crowded_cells()
+    configs.init_fluid_darcy(d, mu=2e-3, k_c=3.5e-13, tolerance=1e-5, maxiter=50, bottom_no_flow=True)
+    path = str(tmp_path / "d.bin")
+    binfile.write_bin(d, path)
+    orc = O.Oracle(path, fluid=True)
+    with Engine(path, fluid=True, precision="faithful") as e:
+        for _ in range(3):
+            assert e.step(1) >= 0
+            assert orc.step(1) == 0, orc.error()
+            phi = numpy.ravel(orc.get("darcy_phi"))
+            assert (phi < 0.6).sum() > 40
+            assert numpy.abs(numpy.ravel(e.get("darcy_phi")) - phi).max() <= 1e-13
+
+
+def test_ns_porosity_of_crowded_cells():
+    from sphere_b200.engine import Engine
+    d = crowded_cells()
+    configs.init_fluid_ns(d, mu=8.9e-4, hydrostatic=True, tolerance=1e-6, maxiter=50)
+    nx, ny, nz = (int(v) for v in d.num)
+    cell = d.L / d.num
+    R = cell.min()
+    volume = 4.0 / 3.0 * 3.14159265358979 * R ** 3
+    ref = numpy.empty((nz, ny, nx))
+    for z in range(nz):
+        for y in range(ny):
+            for x in range(nx):
+                X = numpy.array([x, y, z]) * cell + 0.5 * cell
+                solid = 0.0
+                for sx in (-1, 0, 1):
+                    for sy in (-1, 0, 1):
+                        dist = X - d.x + numpy.array([sx, sy, 0]) * d.L
+                        r = d.radius
+                        # vector lengths are single precision
+                        l = numpy.sqrt((dist ** 2).sum(axis=1).astype(numpy.float32)).astype(numpy.float64)
+                        part = (R - r < l) & (l < R + r)
+                        lens = numpy.pi * (R + r - l) ** 2 * (l * l + 2 * l * r - 3 * r * r + 2 * l * R + 6 * r * R -
+                                                              3 * R * R) / (12.0 * l)
+                        solid += lens[part].sum() + (4.0 / 3.0 * numpy.pi * r ** 3)[l <= R - r].sum()
+                ref[z, y, x] = min(1.0, max(0.0, (volume - solid) / volume))
+    assert (ref < 0.6).sum() > 40
+    with Engine(d, fluid=True, precision="faithful") as e:
+        assert e.step(1) >= 0
+        phi = numpy.ravel(e.get("darcy_phi"))
+        # single-precision lengths: a last-bit difference of one of them shows
+        assert numpy.abs(phi - numpy.ravel(ref)).max() <= 1e-7
+
+
 # one launch per step: re-sorts inside it, the walls one launch behind, calls of
 # one odd length replayed from a graph on either view
 @pytest.mark.parametrize("n,model", [(400, 2), (5000, 1)])
