@@ -89,15 +89,20 @@ typedef struct sph_opts {
                              then wait for a value that nothing writes and give up
                              after about a thousand polls, so the step returns
                              SPH_ERR_TIMEOUT; this exercises the timeout path without
-                             a GPU fault.  An engine that timed out is closed. */
+                             a GPU fault.  An engine that timed out is closed.
+                             SPH_INJECT_GRAPH fails on the host instead and changes
+                             no result */
 } sph_opts;
 
-/* Kernels whose waits sph_opts.inject_timeout makes time out. */
+/* Kernels whose waits sph_opts.inject_timeout makes time out, and a host call
+ * that it makes fail. */
 enum {
     SPH_INJECT_RESORT = 1,     /* the grid barrier of the cooperative cell re-sort */
     SPH_INJECT_PERSISTENT = 2, /* the group barrier of the fused persistent step */
     SPH_INJECT_DARCY = 4,      /* the neighbour waits of the Darcy Jacobi kernel */
     SPH_INJECT_NS = 8,         /* the barrier and waits of the Navier-Stokes Jacobi kernel */
+    SPH_INJECT_GRAPH = 16,     /* CUDA graphs cannot be instantiated (device memory short,
+                                  say): the steps are launched one by one */
 };
 
 /* Fields for sph_get/sph_set.  Vector fields use the reference's Float4

@@ -27,8 +27,9 @@ enum DevErr : int {
 // Fault injection for tests (sph_opts.inject_timeout, values equal to
 // SPH_INJECT_*): the bounded waits of the selected kernels wait for a value
 // nothing writes and give up after kInjectPolls polls, so the error path of a
-// timed-out wait runs without a real hang.
-constexpr uint32_t kInjectResort = 1, kInjectPersistent = 2, kInjectDarcy = 4, kInjectNS = 8;
+// timed-out wait runs without a real hang.  kInjectGraph is host-side: no CUDA
+// graph can be instantiated, so every step is launched by itself.
+constexpr uint32_t kInjectResort = 1, kInjectPersistent = 2, kInjectDarcy = 4, kInjectNS = 8, kInjectGraph = 16;
 constexpr unsigned kInjectPolls = 1u << 10;
 
 // Per-run constants, passed to every kernel by value.

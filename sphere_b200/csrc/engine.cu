@@ -431,8 +431,9 @@ int Engine::ensure_graph()
     return ST_OK;
 }
 
-// A CUDA graph of k per-stage DEM steps on the current state view, or null
-// when capture or instantiation fails (the caller then steps eagerly).
+// A CUDA graph of k per-stage DEM steps from the current state view, or null
+// when capture or instantiation fails (the caller then steps eagerly).  Nothing
+// has run: the current view is the one before, whatever k is.
 cudaGraphExec_t Engine::capture_steps(int k)
 {
     cudaGraph_t g = nullptr;
@@ -442,15 +443,13 @@ cudaGraphExec_t Engine::capture_steps(int k)
     if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
     e = enqueue_steps((uint64_t)k);
     cudaError_t e2 = cudaStreamEndCapture(stream, &g);
-    if (e != cudaSuccess || e2 != cudaSuccess || !g) {
-        if (g) cudaGraphDestroy(g);
-        cudaGetLastError();
-        cur_view = view0;
-        S = S_view[cur_view];
-        return nullptr;
-    }
-    e = cudaGraphInstantiate(&x, g, 0);
-    cudaGraphDestroy(g);
+    cur_view = view0;
+    S = S_view[cur_view];
+    if (e == cudaSuccess && e2 == cudaSuccess && g)
+        e = (inject & kInjectGraph) ? cudaErrorMemoryAllocation : cudaGraphInstantiate(&x, g, 0);
+    else
+        e = cudaErrorUnknown;
+    if (g) cudaGraphDestroy(g);
     if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
     return x;
 }
@@ -485,18 +484,20 @@ int Engine::step_stages(uint64_t n)
     if (n >= 4 && n <= 4 * glen && n != glen && graph_steps > 1 && !graph_failed) {
         ShortGraph &g = short_graph[cur_view];
         const bool seen = g.n == n && g.fused == fused;
-        if (!seen && g.exec) {
-            cudaGraphExecDestroy(g.exec);
-            g.exec = nullptr;
+        if (!seen) {
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            g = ShortGraph();
+            g.n = n;
+            g.fused = fused;
         }
-        g.n = n;
-        g.fused = fused;
-        const bool odd = fused && (n & 1);
-        if (seen && !g.exec && (g.exec = capture_steps((int)n)) && odd) flip_view();   // capturing flipped it
+        if (seen && !g.exec && !g.failed) {
+            g.exec = capture_steps((int)n);
+            g.failed = !g.exec;
+        }
         if (g.exec) {
             cudaError_t e = cudaGraphLaunch(g.exec, stream);
             if (e != cudaSuccess) return cuda_fail(e, "graph launch");
-            if (odd) flip_view();
+            if (fused && (n & 1)) flip_view();
             advance_host_clock(n);
             return poll_errors("step");
         }
@@ -863,7 +864,8 @@ int Engine::run()
 }  // namespace sphb
 
 static_assert(sphb::kInjectResort == SPH_INJECT_RESORT && sphb::kInjectPersistent == SPH_INJECT_PERSISTENT &&
-                  sphb::kInjectDarcy == SPH_INJECT_DARCY && sphb::kInjectNS == SPH_INJECT_NS,
+                  sphb::kInjectDarcy == SPH_INJECT_DARCY && sphb::kInjectNS == SPH_INJECT_NS &&
+                  sphb::kInjectGraph == SPH_INJECT_GRAPH,
               "fault-injection bits of the device code and the C ABI");
 
 using sphb::Engine;

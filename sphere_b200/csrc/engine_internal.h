@@ -68,6 +68,7 @@ public:
         cudaGraphExec_t exec = nullptr;
         uint64_t n = 0;
         bool fused = false;
+        bool failed = false;   // could not be made: not tried again for this n
     };
     ShortGraph short_graph[2];
     bool warmed = false;

@@ -52,7 +52,7 @@ class SphOpts(ctypes.Structure):
 
 
 # sph_opts.inject_timeout bits (SPH_INJECT_*)
-INJECT = {"resort": 1, "persistent": 2, "darcy": 4, "ns": 8}
+INJECT = {"resort": 1, "persistent": 2, "darcy": 4, "ns": 8, "graph": 16}
 
 
 class SphInfo(ctypes.Structure):

@@ -196,6 +196,24 @@ def test_one_launch_steps_with_resorts(tmp_path, n, model):
         assert e.info().resorts > 5
 
 
+# graphs that cannot be instantiated: calls of an odd length step one by one from
+# the buffer that holds the state
+@pytest.mark.parametrize("kernel,steps", [("stages_fused", (3, 5, 5, 5, 5, 6, 6)), ("auto", (5, 5, 5, 5, 5, 150)),
+                                          ("stages", (5, 5, 5))])
+def test_steps_without_graphs(tmp_path, kernel, steps):
+    from sphere_b200.engine import Engine
+    d = pressed(400)
+    path = str(tmp_path / "nograph.bin")
+    binfile.write_bin(d, path)
+    orc = O.Oracle(path)
+    with Engine(path, step_kernel=kernel, inject_timeout="graph") as e:
+        for n in steps:
+            assert orc.step(n) == 0, orc.error()
+            assert e.step(n) == 0
+            bad = compare(e, orc)
+            assert not bad, (n, bad)
+
+
 # more neighbours than a list holds (48): the particle scans the cells instead
 @pytest.mark.parametrize("model", [1, 2])
 def test_full_neighbour_list(tmp_path, model):
