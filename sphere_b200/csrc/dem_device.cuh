@@ -4,6 +4,8 @@
 // dem_kernels.cu (compiled with -fmad=false), the mixed one in dem_mixed.cu.
 #pragma once
 
+#include <type_traits>
+
 #include "dem_state.h"
 #include "reduce_device.cuh"
 #include "resort_device.cuh"
@@ -549,7 +551,8 @@ __device__ __forceinline__ bool touches(const DevParams &P, const double4 &xa, c
 // PREC 0: faithful FP64, 1: FP64, 2: mixed (FP64 overlap, FP32 contact law,
 // FP64 accumulation).
 // before_walls() runs in all lanes once the contacts are done and before the
-// walls are read.
+// walls are read.  With one (k_step) a capacity error is raised after it: the
+// step before is complete by then, so an error never reaches back to it.
 struct WallsReady {
     __device__ __forceinline__ void operator()() const {}
 };
@@ -560,6 +563,12 @@ __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState 
 {
     constexpr int TP = PREC == 2 ? 1 : PREC;  // precision of overlap tests
     constexpr unsigned ALL = 0xffffffffu;
+    constexpr bool LATE = !std::is_same_v<std::decay_t<Before>, WallsReady>;
+    int over = -1;   // LATE: the particle whose row has no place
+    auto capacity_error = [&](unsigned orig) {
+        if constexpr (LATE) over = (int)orig;
+        else raise_err(S.ctl, DERR_CAPACITY, (int)orig);
+    };
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ip = lane & (pw - 1u), sub = lane / pw, S_ = 32u / pw;
     const unsigned np = P.np, NC = P.nc;
@@ -698,7 +707,7 @@ __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState 
             if (nhit > NC) ok = false;
             if (!ok) {
                 // the row keeps the contacts it had
-                raise_err(S.ctl, DERR_CAPACITY, (int)o);
+                capacity_error(o);
                 for (uint64_t m = mask & ~mask0; m; m &= m - 1)
                     S.contacts[rowbase + (__ffsll((long long)m) - 1)] = np;
             }
@@ -740,7 +749,7 @@ __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState 
                     e = there ? S.pos_of[b_orig] | (uint32_t)S.dmcode[mempos] << 28 : 0u;
                 }
                 if (!there) {
-                    raise_err(S.ctl, DERR_CAPACITY, (int)S.orig_of[ka]);
+                    capacity_error(S.orig_of[ka]);
                 } else {
                     const V3 dm = dm_decode(P, (uint8_t)(e >> 28));
                     const unsigned kb = e & 0x0fffffffu;
@@ -824,6 +833,7 @@ __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState 
         __syncwarp();
     }
     before_walls();
+    if (LATE && over >= 0) raise_err(S.ctl, DERR_CAPACITY, over);
     if (!ok) return false;
     const double4 vel_a = S.vel[k];
     const V3 angvel_a = xyz(S.angvel[k]);

@@ -6,6 +6,7 @@ with a status and a message naming the particle; the engine closes cleanly
 and a new engine on the same device steps normally.  An empty particle set
 steps without error."""
 import numpy
+import numpy
 import pytest
 
 from sphere_b200 import configs
@@ -36,6 +37,35 @@ def test_capacity_overflow_is_reported():
     ok = Engine(d, capacity=32)
     assert ok.step(5) == 0
     ok.close()
+
+
+@pytest.mark.parametrize("shape", [(6, 6, 6), (48, 48, 43)])
+def test_overflow_leaves_the_steps_before_it_whole(shape):
+    """The one-launch step moves the walls of the step before while it searches
+    contacts: a row that overflows in that search must not take the finished
+    step's clock and wall motion along.  Rows of three spheres: the outer two
+    reach the middle one in the same step, which has one slot."""
+    from sphere_b200.engine import Engine, EngineError
+    n = int(numpy.prod(shape))
+    d = configs.settling_lattice(n=n, seed=5, nx=shape[0], ny=shape[1], nz=shape[2], spacing=0.0205,
+                                 jitter=0.0, r_min=0.01, r_max=0.01, steps=100)
+    configs.add_top_wall(d, 10e3)
+    speed = 0.0005 / (8.5 * float(d.time_dt))
+    d.vel = numpy.zeros((n, 3))
+    d.vel[:, 0] = numpy.array([speed, 0.0, -speed])[(numpy.arange(n) % shape[0]) % 3]
+    for _ in range(5):
+        after = []
+        for kernel in ("stages", "stages_fused"):
+            e = Engine(d, capacity=1, step_kernel=kernel)
+            assert e.step(3) == 0
+            with pytest.raises(EngineError) as exc:
+                e.step(20)
+            assert exc.value.status == -6
+            after.append((int(e.get("iter")[0]), float(e.get("time")[0]), e.get("walls_nx").tobytes(),
+                          e.get("walls_mvfd").tobytes()))
+            e.close()
+        assert 4 < after[0][0] < 20
+        assert after[0] == after[1]
 
 
 def test_particle_leaving_the_grid_is_reported():
