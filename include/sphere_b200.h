@@ -103,6 +103,7 @@ enum {
     SPH_INJECT_NS = 8,         /* the barrier and waits of the Navier-Stokes Jacobi kernel */
     SPH_INJECT_GRAPH = 16,     /* CUDA graphs cannot be instantiated (device memory short,
                                   say): the steps are launched one by one */
+    SPH_INJECT_STEP = 32,      /* the waits of the one-launch step, its re-sort's included */
 };
 
 /* Fields for sph_get/sph_set.  Vector fields use the reference's Float4

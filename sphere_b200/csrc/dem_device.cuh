@@ -551,10 +551,11 @@ __device__ __forceinline__ bool touches(const DevParams &P, const double4 &xa, c
 // PREC 0: faithful FP64, 1: FP64, 2: mixed (FP64 overlap, FP32 contact law,
 // FP64 accumulation).
 // before_walls() runs in all lanes once the contacts are done and before the
-// walls are read.  With one (k_step) a capacity error is raised after it: the
+// walls are read; where it returns false (k_step, whose wait ran out) no particle
+// of the warp goes on.  With one, a capacity error is raised after it: the
 // step before is complete by then, so an error never reaches back to it.
 struct WallsReady {
-    __device__ __forceinline__ void operator()() const {}
+    __device__ __forceinline__ bool operator()() const { return true; }
 };
 template <int PREC, int MODEL, class Before = WallsReady>
 __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState &S, unsigned k0,
@@ -832,9 +833,9 @@ __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState 
         }
         __syncwarp();
     }
-    before_walls();
+    const bool go = before_walls();
     if (LATE && over >= 0) raise_err(S.ctl, DERR_CAPACITY, over);
-    if (!ok) return false;
+    if (!ok || !go) return false;
     const double4 vel_a = S.vel[k];
     const V3 angvel_a = xyz(S.angvel[k]);
     if (MODEL == 2) {
@@ -1454,15 +1455,17 @@ k_contacts_integrate(DevParams P, DevState S, unsigned pw)
 }
 
 // Bounded wait of one warp until *p == want (acquire): false after ~2^24 polls
-// (DERR_TIMEOUT), or when another block has timed out.
-__device__ __forceinline__ bool wait_equal(const unsigned *p, unsigned want, DevCtl *ctl)
+// (DERR_TIMEOUT), or when another block has timed out.  With `inject` it never
+// succeeds and gives up after kInjectPolls polls.
+__device__ __forceinline__ bool wait_equal(const unsigned *p, unsigned want, DevCtl *ctl, bool inject)
 {
     unsigned spins = 0;
+    const unsigned limit = inject ? kInjectPolls : 1u << 24;
     for (;;) {
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-        if (v == want) return true;
-        if (++spins > (1u << 24)) {
+        if (v == want && !inject) return true;
+        if (++spins > limit) {
             raise_err(ctl, DERR_TIMEOUT, -1);
             return false;
         }
@@ -1500,6 +1503,7 @@ k_step(DevParams P, DevState S, PermScratch W, unsigned pw, int view, int pendin
     constexpr unsigned ALL = 0xffffffffu;
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     DevCtl *ctl = S.ctl;
+    const bool inject = (P.inject & kInjectStep) != 0;
     const unsigned stamp = __ldcg(&ctl->stamp[view]);
     const bool err = __shfl_sync(ALL, *(volatile int *)&ctl->err, 0) != 0;
     const bool resort = pending ? __ldcg(&ctl->resort_at[view]) == (int)stamp : __ldcg(&ctl->resort) != 0;
@@ -1518,14 +1522,14 @@ k_step(DevParams P, DevState S, PermScratch W, unsigned pw, int view, int pendin
         }
     }
     if (resort && !err) {
-        auto bar = [&]() { return grid_barrier(ctl, gridDim.x, (P.inject & kInjectResort) != 0); };
+        auto bar = [&]() { return grid_barrier(ctl, gridDim.x, inject); };
         if (!resort_group(P, S, W, gridDim.x, blockIdx.x, bar, true) || !bar()) return;
     }
     if (blockIdx.x == 0) {
         if (warp != 0) return;
         if (pending) {
             const unsigned summing = min(nb, nchunks);
-            if (!__all_sync(ALL, wait_equal(&ctl->ticket, summing, ctl))) return;
+            if (!__all_sync(ALL, wait_equal(&ctl->ticket, summing, ctl, inject))) return;
             advance_walls(P, S);
         }
         if (lane == 0) {
@@ -1550,8 +1554,9 @@ k_step(DevParams P, DevState S, PermScratch W, unsigned pw, int view, int pendin
     }
     const WarpScratch ws = contact_warp_scratch<PREC, MODEL>(contact_smem, warp, P.nc);
     auto walls = [&] {
-        if (pending) (void)wait_equal(&ctl->ready, stamp, ctl);
+        const bool moved = !pending || wait_equal(&ctl->ready, stamp, ctl, inject);
         __syncwarp();
+        return __all_sync(ALL, moved) != 0;
     };
     if (!contacts_integrate_warp<PREC, MODEL, false>(P, S, k0, pw, ws, [&] { return read_clock(ctl); },
                                               StepFlags{&ctl->resort_at[view ^ 1], &ctl->nl_at[view ^ 1],

@@ -29,7 +29,8 @@ enum DevErr : int {
 // nothing writes and give up after kInjectPolls polls, so the error path of a
 // timed-out wait runs without a real hang.  kInjectGraph is host-side: no CUDA
 // graph can be instantiated, so every step is launched by itself.
-constexpr uint32_t kInjectResort = 1, kInjectPersistent = 2, kInjectDarcy = 4, kInjectNS = 8, kInjectGraph = 16;
+constexpr uint32_t kInjectResort = 1, kInjectPersistent = 2, kInjectDarcy = 4, kInjectNS = 8, kInjectGraph = 16,
+                   kInjectStep = 32;
 constexpr unsigned kInjectPolls = 1u << 10;
 
 // Per-run constants, passed to every kernel by value.

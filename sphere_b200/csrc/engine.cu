@@ -865,7 +865,7 @@ int Engine::run()
 
 static_assert(sphb::kInjectResort == SPH_INJECT_RESORT && sphb::kInjectPersistent == SPH_INJECT_PERSISTENT &&
                   sphb::kInjectDarcy == SPH_INJECT_DARCY && sphb::kInjectNS == SPH_INJECT_NS &&
-                  sphb::kInjectGraph == SPH_INJECT_GRAPH,
+                  sphb::kInjectGraph == SPH_INJECT_GRAPH && sphb::kInjectStep == SPH_INJECT_STEP,
               "fault-injection bits of the device code and the C ABI");
 
 using sphb::Engine;

@@ -52,7 +52,7 @@ class SphOpts(ctypes.Structure):
 
 
 # sph_opts.inject_timeout bits (SPH_INJECT_*)
-INJECT = {"resort": 1, "persistent": 2, "darcy": 4, "ns": 8, "graph": 16}
+INJECT = {"resort": 1, "persistent": 2, "darcy": 4, "ns": 8, "graph": 16, "step": 32}
 
 
 class SphInfo(ctypes.Structure):

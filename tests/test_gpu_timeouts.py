@@ -2,9 +2,10 @@
 
 Every cooperative kernel of the engine waits on other blocks through bounded
 polls (the cell re-sort's grid barrier, the fused step's group barrier, the
-neighbour waits of the Darcy and Navier-Stokes Jacobi kernels).  With
-sph_opts.inject_timeout the selected kernel's waits target a value that
-nothing writes and give up after about a thousand polls: the kernel returns,
+one-launch step's wait for its walls, the neighbour waits of the Darcy and
+Navier-Stokes Jacobi kernels).  With sph_opts.inject_timeout the selected
+kernel's waits target a value that nothing writes and give up after about a
+thousand polls: the kernel returns,
 the call reports SPH_ERR_TIMEOUT (-9) and the GPU context stays usable.  Each
 test then checks that an engine opened afterwards on the same device steps
 exactly like one opened before the timeout (and, for the DEM, like the
@@ -85,6 +86,41 @@ def test_persistent_group_barrier_timeout(tmp_path):
     assert ei.value.status == TIMEOUT
     eng.close()
     check_dem_after(tmp_path, d, before, "persistent")
+
+
+def test_one_launch_step_wait_timeout():
+    """The first step of a call has nothing to wait for; in the second the wait
+    for its walls runs out.  It must not go on without them: every particle
+    stays at the end of the first."""
+    from sphere_b200.engine import Engine, EngineError
+    d = dem_box(5)
+    eng = Engine(d, step_kernel="stages_fused", inject_timeout="step")
+    assert eng.step(1) == 0      # three launches: no wait of the one-launch step
+    with pytest.raises(EngineError) as ei:
+        eng.step(6)
+    assert ei.value.status == TIMEOUT
+    got = {f: numpy.array(eng.get(f), copy=True) for f in ("x", "vel", "angvel")}
+    eng.close()
+    same_bits(got, run_fields(lambda: Engine(d, step_kernel="stages"), (2,), ("x", "vel", "angvel")))
+
+
+def test_one_launch_step_resort_barrier_timeout(tmp_path):
+    from sphere_b200.engine import Engine, EngineError
+    d = dem_box(6)
+    before = run_fields(lambda: Engine(d, step_kernel="stages_fused"), (3, 9), DEM_FIELDS)
+    moving = dem_box(6)
+    moving.vel = moving.vel + numpy.random.default_rng(8).uniform(-200.0, 200.0, size=moving.vel.shape)
+    eng = Engine(moving, step_kernel="stages_fused", inject_timeout="step")
+    for _ in range(200):         # calls of one step: nothing to wait for but a re-sort
+        try:
+            assert eng.step(1) == 0
+        except EngineError as err:
+            assert err.status == TIMEOUT
+            break
+    else:
+        raise AssertionError("no sphere changed its cell")
+    eng.close()
+    check_dem_after(tmp_path, d, before, "stages_fused")
 
 
 def darcy_box(seed=51):
