@@ -177,8 +177,9 @@ typedef struct sph_info {
     int32_t step_path;    /* 0 per-stage kernels, 1 fused persistent step, 2 per-stage
                              kernels with contacts and integration in one launch (the
                              whole step in one where the system fits one wave) */
-    int32_t step_threads; /* persistent path: threads per block chosen by the autotuner */
-    int32_t step_grid;    /* persistent path: blocks of the launch */
+    int32_t step_threads; /* persistent path: threads per block chosen by the autotuner;
+                             0 on the others */
+    int32_t step_grid;    /* persistent path: blocks of the launch; 0 on the others */
     int32_t tuned;        /* 1 once the autotuner has run */
 } sph_info;
 

@@ -160,9 +160,12 @@ void *Engine::persist_ctl() const { return persist ? (void *)persist->pc : nullp
 
 void Engine::persist_describe(sph_info *info) const
 {
-    info->step_path = (persist && !persist_off) ? 1 : (fused ? 2 : 0);
-    info->step_threads = persist ? kPersistShapes[persist->shape].threads : 0;
-    info->step_grid = persist ? (int32_t)persist->grid : 0;
+    // an automatic engine steps with the persistent kernel only once the tuner
+    // has chosen it
+    const bool persistent = persist && !persist_off && (persist->tuned || step_kernel == 2);
+    info->step_path = persistent ? 1 : ((fused || (persist && !persist_off)) ? 2 : 0);
+    info->step_threads = persistent ? kPersistShapes[persist->shape].threads : 0;
+    info->step_grid = persistent ? (int32_t)persist->grid : 0;
     info->tuned = persist ? (persist->tuned ? 1 : 0) : 0;
 }
 

@@ -214,6 +214,22 @@ def test_steps_without_graphs(tmp_path, kernel, steps):
             assert not bad, (n, bad)
 
 
+def test_reported_step_path():
+    from sphere_b200.engine import Engine
+    d = pressed(400)
+    shape = lambda i: (i.step_path, i.step_threads > 0, i.step_grid > 0, i.tuned)  # noqa: E731
+    for kernel, path in (("stages", 0), ("persistent", 1), ("stages_fused", 2)):
+        with Engine(d, step_kernel=kernel) as e:
+            e.step(5)
+            assert shape(e.info())[:3] == (path, path == 1, path == 1)
+    with Engine(d) as e:
+        e.step(5)                      # too short to tune on
+        assert shape(e.info()) == (2, False, False, 0)
+        e.step(400)
+        path, threads, grid, tuned = shape(e.info())
+        assert tuned == 1 and threads == grid == (path == 1)
+
+
 # more neighbours than a list holds (48): the particle scans the cells instead
 @pytest.mark.parametrize("model", [1, 2])
 def test_full_neighbour_list(tmp_path, model):
