@@ -955,13 +955,19 @@ __device__ __forceinline__ void nl_build_particle(const DevParams &P, const DevS
     const double ra = xa.w;
     unsigned n = 0;
     const size_t np = P.np;
+    // a remembered slot that the row confirms is the partner's first slot unless
+    // the row names it twice; no row that the engine has built does
+    const bool forget = S.ctl->rows_twice != 0;
     for_each_cell_candidate(P, S, k, xa, [&](unsigned b, int sx, int sy) {
         double4 xb = S.x[b];
         V3 dm = shift_vec(P, sx, sy);
         V3 xab = add3(mk3(xa.x - xb.x, xa.y - xb.y, xa.z - xb.z), dm);
         double reach = ra + xb.w + P.skin;
         if (dot3(xab, xab) < reach * reach) {
-            if (n < P.nlmax) S.nl[(size_t)n * np + k] = b | ((uint32_t)dm_encode(sx, sy) << 28);
+            if (n < P.nlmax) {
+                S.nl[(size_t)n * np + k] = b | ((uint32_t)dm_encode(sx, sy) << 28);
+                if (forget) S.nl_slot[(size_t)n * np + k] = kNoSlot;
+            }
             ++n;
         }
         return true;

@@ -17,8 +17,13 @@ __global__ void k_occ_from_rows(DevParams P, DevState S)
     unsigned o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= P.np) return;
     uint64_t m = 0;
+    const uint32_t *row = S.contacts + (size_t)o * P.nc;
     for (unsigned i = 0; i < P.nc; ++i)
-        if (S.contacts[(size_t)o * P.nc + i] != P.np) m |= 1ull << i;
+        if (row[i] != P.np) {
+            m |= 1ull << i;
+            for (unsigned j = 0; j < i; ++j)
+                if (row[j] == row[i]) S.ctl->rows_twice = 1;
+        }
     S.occ[o] = m;
 }
 // ---------------------------------------------------------------------

@@ -13,6 +13,8 @@
 
 namespace sphb {
 
+constexpr uint8_t kNoSlot = 0xff;
+
 struct DevState {
     // sorted particle storage (the reference's Float4 layout per particle)
     double4 *x, *vel, *angvel, *angpos, *acc, *angacc, *xyzsum, *force, *torque;
@@ -42,7 +44,8 @@ struct DevState {
     // = sorted index | periodic shift code << 28
     uint32_t *nl, *nl_count;
     // slot that the partner of list entry j of particle k last had in k's row
-    // (nl_slot[j*np + k]): a hint, valid only where the row confirms it
+    // (nl_slot[j*np + k]): a hint, valid only where the row confirms it; kNoSlot
+    // remembers none
     uint8_t *nl_slot;
     float4 *x_ref;         // position at the last list build
 

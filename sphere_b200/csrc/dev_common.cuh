@@ -82,6 +82,7 @@ struct DevCtl {
     int resort_at[2];
     int nl_at[2];
     unsigned ready;
+    int rows_twice;            // 1: the caller's rows name a partner twice
 };
 
 struct V3 {

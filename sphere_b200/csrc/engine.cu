@@ -683,7 +683,10 @@ int Engine::set(int f, const void *src, size_t bytes)
         switch (f) {
         case SPH_F_CONTACTS:
             e = cudaMemcpyAsync(S.contacts, src, bytes, cudaMemcpyHostToDevice, stream);
+            if (e == cudaSuccess) e = cudaMemsetAsync(&S.ctl->rows_twice, 0, sizeof(int), stream);
             if (e == cudaSuccess) e = launch_occ_from_rows(P, S, stream);
+            // the slots that the lists remember belong to the rows before
+            if (e == cudaSuccess) e = cudaMemsetAsync(S.nl_slot, kNoSlot, n * (size_t)nlmax, stream);
             break;
         case SPH_F_DELTA_T:
             if (S.delta_t_f) {

@@ -214,6 +214,34 @@ def test_steps_without_graphs(tmp_path, kernel, steps):
             assert not bad, (n, bad)
 
 
+# rows set by the caller that name a partner twice: the first of its slots is the
+# one that takes this step's periodic shift, whatever slot it had before; with
+# velocities so that particles change places in the sort meanwhile
+@pytest.mark.parametrize("kernel", ["stages", "stages_fused", "persistent"])
+def test_rows_with_a_partner_twice(tmp_path, kernel):
+    from sphere_b200.engine import Engine
+    d = pressed(400)
+    d.vel = numpy.random.default_rng(7).uniform(-20.0, 20.0, size=(d.np, 3))
+    path = str(tmp_path / "twice.bin")
+    binfile.write_bin(d, path)
+    orc = O.Oracle(path)
+    with Engine(path, step_kernel=kernel) as e:
+        assert orc.step(5) == 0 and e.step(5) == 0
+        rows = e.get("contacts").reshape(d.np, -1)
+        shift = e.get("distmod").reshape(d.np, -1, 4)
+        assert (numpy.abs(shift[:, -1, :2]).sum(axis=1) > 0).sum() > 10
+        rows[:, 0] = rows[:, -1]
+        orc.set("contacts", rows)
+        e.set("contacts", rows)
+        before = e.info().resorts
+        for steps in (1, 4, 25):
+            assert orc.step(steps) == 0, orc.error()
+            assert e.step(steps) == 0
+            bad = compare(e, orc)
+            assert not bad, (steps, bad)
+        assert e.info().resorts > before + 3
+
+
 def test_reported_step_path():
     from sphere_b200.engine import Engine
     d = pressed(400)
