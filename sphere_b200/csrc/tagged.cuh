@@ -1,7 +1,7 @@
-// Cell values that carry the iteration they belong to, for the fluid solvers'
-// Jacobi kernels.
+// Cell values that carry the iteration they belong to, for the Darcy solver's
+// Jacobi kernel.
 //
-// An iteration of those kernels is a few hundred nanoseconds of arithmetic per
+// An iteration of that kernel is a few hundred nanoseconds of arithmetic per
 // cell, so its cost is the hand-over of the iterates between thread blocks.
 // With a flag per block that hand-over is a fence, a store, a poll, a block
 // barrier and then the loads; here the value is its own flag: a cell's new
@@ -70,13 +70,13 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
 // correction rounds as the division does; the first correction brings the
 // quotient within one unit).  Operands outside the range in which the
 // remainders are exact take the division.
-__device__ __forceinline__ double div_by(double x, double d, double r)
+__host__ __device__ __forceinline__ double div_by(double x, double d, double r)
 {
     const double a = fabs(x);
     if (!(a > 1e-200 && a < 1e200)) return x / d;
     double q = x * r;
-    q = __fma_rn(__fma_rn(-q, d, x), r, q);
-    return __fma_rn(__fma_rn(-q, d, x), r, q);
+    q = fma(fma(-q, d, x), r, q);
+    return fma(fma(-q, d, x), r, q);
 }
 
 }  // namespace sphb
