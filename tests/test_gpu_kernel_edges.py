@@ -9,7 +9,8 @@
   against the renderer that tests every sphere.
 * One launch per step, with re-sorts inside it, against the oracle.
 * The Darcy iteration keeps one, two or four cells per thread in registers and
-  leaves out those that cannot change.
+  leaves out those that cannot change: both sides of each of its limits, and of
+  the largest grid it takes.
 """
 import numpy
 import pytest
@@ -90,8 +91,8 @@ def test_render_tiles_with_many_spheres(n, scale):
                 assert numpy.array_equal(img[:, :, :3], ref[:, :, :3]), (n, w, h)
 
 
-# cells that change: one, two or four per thread of the solver's 148 x 256
-# threads, and a lid of cells that stay as they are
+# a lid of cells that stay as they are, and none; one cell per thread of the
+# solver's 148 x 256 threads, and four
 @pytest.mark.parametrize("grid,lid", [((8, 8, 9), 2), ((33, 35, 32), 0), ((40, 40, 60), 3), ((40, 40, 80), 0)])
 def test_darcy_cells_per_thread(tmp_path, grid, lid):
     from sphere_b200.engine import Engine
@@ -115,6 +116,39 @@ def test_darcy_cells_per_thread(tmp_path, grid, lid):
             for f in ("darcy_p", "darcy_v", "darcy_phi"):
                 a, b = numpy.ravel(e.get(f)), numpy.ravel(orc.get(f))
                 assert numpy.abs(a - b).max() <= RTOL * max(numpy.abs(b).max(), 1e-300), f
+
+
+# layers of 1184 = 148 x 8 cells, the top one fixed: a block of the solver takes 256
+# changing cells with one per thread, 512 with two, 1024 with four; beyond 148 x
+# 1024 cells in all k_jacobi runs.  Pressures that differ in every cell
+@pytest.mark.parametrize("nz,per_thread", [(33, 1), (34, 2), (65, 2), (66, 4), (128, 4), (129, None)])
+def test_darcy_cells_per_thread_limits(tmp_path, nz, per_thread):
+    import torch
+    from sphere_b200.engine import Engine
+    from test_gpu_darcy import RTOL
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if sms != 148:
+        pytest.skip("the limits are those of 148 SMs")
+    grid = (37, 32, nz)
+    cells, active = 1184 * nz, 1184 * (nz - 1)
+    chunk = (-(-active // sms) + 31) // 32 * 32
+    assert per_thread == (None if cells > sms * 1024 else 1 if chunk <= 256 else 2 if chunk <= 512 else 4)
+    d = configs.settling_lattice(n=300, seed=51, nx=7, ny=7, nz=7, spacing=0.0195, steps=40)
+    d.num = numpy.array(grid, dtype=numpy.uint32)
+    d.L = numpy.array(grid) * 0.024
+    configs.init_fluid_darcy(d, mu=2e-3, k_c=3.5e-13, tolerance=1e-7, maxiter=45, bottom_no_flow=True)
+    d.p_f[:, :, :-1] = numpy.random.default_rng(nz).uniform(1e3, 2e3, size=d.p_f[:, :, :-1].shape)
+    path = str(tmp_path / "d.bin")
+    binfile.write_bin(d, path)
+    orc = O.Oracle(path, fluid=True)
+    with Engine(path, fluid=True, precision="faithful") as e:
+        for _ in range(2):
+            assert e.step(1) >= 0
+            assert orc.step(1) == 0, orc.error()
+            assert int(e.get("darcy_iters")[0]) == int(orc.get("darcy_nijac_last")[0]) > 30
+            for f in ("darcy_p", "darcy_v"):
+                a, b = numpy.ravel(e.get(f)), numpy.ravel(orc.get(f))
+                assert numpy.abs(a - b).max() <= RTOL * numpy.abs(b).max(), f
 
 
 def crowded_cells():
