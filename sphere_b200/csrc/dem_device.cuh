@@ -552,7 +552,7 @@ __device__ __forceinline__ bool touches(const DevParams &P, const double4 &xa, c
 // FP64 accumulation).
 // before_walls() runs in all lanes once the contacts are done and before the
 // walls are read; where it returns false (k_step, whose wait ran out) no particle
-// of the warp goes on.  With one, a capacity error is raised after it: the
+// of the warp goes on.  With one, the error of a full row is raised after it: the
 // step before is complete by then, so an error never reaches back to it.
 struct WallsReady {
     __device__ __forceinline__ bool operator()() const { return true; }
@@ -565,11 +565,6 @@ __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState 
     constexpr int TP = PREC == 2 ? 1 : PREC;  // precision of overlap tests
     constexpr unsigned ALL = 0xffffffffu;
     constexpr bool LATE = !std::is_same_v<std::decay_t<Before>, WallsReady>;
-    int over = -1;   // LATE: the particle whose row has no place
-    auto capacity_error = [&](unsigned orig) {
-        if constexpr (LATE) over = (int)orig;
-        else raise_err(S.ctl, DERR_CAPACITY, (int)orig);
-    };
     const unsigned lane = threadIdx.x & 31u;
     const unsigned ip = lane & (pw - 1u), sub = lane / pw, S_ = 32u / pw;
     const unsigned np = P.np, NC = P.nc;
@@ -708,7 +703,7 @@ __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState 
             if (nhit > NC) ok = false;
             if (!ok) {
                 // the row keeps the contacts it had
-                capacity_error(o);
+                if (!LATE) raise_err(S.ctl, DERR_CAPACITY, (int)o);
                 for (uint64_t m = mask & ~mask0; m; m &= m - 1)
                     S.contacts[rowbase + (__ffsll((long long)m) - 1)] = np;
             }
@@ -750,7 +745,8 @@ __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState 
                     e = there ? S.pos_of[b_orig] | (uint32_t)S.dmcode[mempos] << 28 : 0u;
                 }
                 if (!there) {
-                    capacity_error(S.orig_of[ka]);
+                    // a partner that the caller's row names: the first step of a call
+                    raise_err(S.ctl, DERR_CAPACITY, (int)S.orig_of[ka]);
                 } else {
                     const V3 dm = dm_decode(P, (uint8_t)(e >> 28));
                     const unsigned kb = e & 0x0fffffffu;
@@ -834,7 +830,7 @@ __device__ __forceinline__ bool contact_warp(const DevParams &P, const DevState 
         __syncwarp();
     }
     const bool go = before_walls();
-    if (LATE && over >= 0) raise_err(S.ctl, DERR_CAPACITY, over);
+    if (MODEL == 2 && LATE && owner && !ok) raise_err(S.ctl, DERR_CAPACITY, (int)S.orig_of[k]);
     if (!ok || !go) return false;
     const double4 vel_a = S.vel[k];
     const V3 angvel_a = xyz(S.angvel[k]);
