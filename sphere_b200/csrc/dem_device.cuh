@@ -551,8 +551,8 @@ __device__ __forceinline__ bool touches(const DevParams &P, const double4 &xa, c
 // PREC 0: faithful FP64, 1: FP64, 2: mixed (FP64 overlap, FP32 contact law,
 // FP64 accumulation).
 // before_walls() runs in all lanes once the contacts are done and before the
-// walls are read; where it returns false (k_step, whose wait ran out) no particle
-// of the warp goes on.  With one, the error of a full row is raised after it: the
+// walls are read; where it returns false (k_step, whose wait ran out) the lane's
+// particle does not go on.  With one, the error of a full row is raised after it: the
 // step before is complete by then, so an error never reaches back to it.
 struct WallsReady {
     __device__ __forceinline__ bool operator()() const { return true; }
@@ -1456,17 +1456,16 @@ k_contacts_integrate(DevParams P, DevState S, unsigned pw)
         carry_particle(S, k);
 }
 
-// Bounded wait of one warp until *p == want (acquire): false after ~2^24 polls
-// (DERR_TIMEOUT), or when another block has timed out.  With `inject` it never
-// succeeds and gives up after kInjectPolls polls.
-__device__ __forceinline__ bool wait_equal(const unsigned *p, unsigned want, DevCtl *ctl, bool inject)
+// Bounded wait of one warp until *p == want (acquire): false after `limit` polls
+// (DERR_TIMEOUT), or when another block has timed out.
+__device__ __forceinline__ bool wait_equal(const unsigned *p, unsigned want, DevCtl *ctl,
+                                           unsigned limit = 1u << 24)
 {
     unsigned spins = 0;
-    const unsigned limit = inject ? kInjectPolls : 1u << 24;
     for (;;) {
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-        if (v == want && !inject) return true;
+        if (v == want) return true;
         if (++spins > limit) {
             raise_err(ctl, DERR_TIMEOUT, -1);
             return false;
@@ -1530,8 +1529,10 @@ k_step(DevParams P, DevState S, PermScratch W, unsigned pw, int view, int pendin
     if (blockIdx.x == 0) {
         if (warp != 0) return;
         if (pending) {
-            const unsigned summing = min(nb, nchunks);
-            if (!__all_sync(ALL, wait_equal(&ctl->ticket, summing, ctl, inject))) return;
+            // (injected: a count that is never reached, and the others, whose
+            // word then never comes, stop at this block's error)
+            const unsigned summing = inject ? ~0u : min(nb, nchunks);
+            if (!__all_sync(ALL, wait_equal(&ctl->ticket, summing, ctl, inject ? kInjectPolls : 1u << 24))) return;
             advance_walls(P, S);
         }
         if (lane == 0) {
@@ -1556,9 +1557,9 @@ k_step(DevParams P, DevState S, PermScratch W, unsigned pw, int view, int pendin
     }
     const WarpScratch ws = contact_warp_scratch<PREC, MODEL>(contact_smem, warp, P.nc);
     auto walls = [&] {
-        const bool moved = !pending || wait_equal(&ctl->ready, stamp, ctl, inject);
+        const bool moved = !pending || wait_equal(&ctl->ready, stamp, ctl);
         __syncwarp();
-        return __all_sync(ALL, moved) != 0;
+        return moved;
     };
     if (!contacts_integrate_warp<PREC, MODEL, false>(P, S, k0, pw, ws, [&] { return read_clock(ctl); },
                                               StepFlags{&ctl->resort_at[view ^ 1], &ctl->nl_at[view ^ 1],
