@@ -138,6 +138,21 @@ def step_path_name(info):
         int(info.step_path), "per-stage")
 
 
+def timed_launches(info, d, steps):
+    """Launches of this library's kernels in `steps` timed benchmark steps.
+    Persistent path: one k_persistent per call.  Contacts and integration in one
+    launch, systems of one wave, as the shear workload: one k_step per DEM step
+    and a k_step_end per call.  Per-stage path: k_resort (with the list rebuild),
+    k_contacts and k_integrate per DEM step (+2 for the shear-stress wall, +2
+    with bonds)."""
+    if info.step_path == 1:
+        return steps
+    if info.step_path == 2:
+        return (INTERVAL + 1) * steps
+    per_step = 3 + (2 if d.nw > 0 and d.wmode[0] == 3 else 0) + (2 if d.nb0 > 0 else 0)
+    return per_step * INTERVAL * steps
+
+
 def mean_contacts(eng, n):
     c = eng.get("contacts")
     return float((c != n).sum()) / n
@@ -281,22 +296,13 @@ def run_gpu(args):
         # angvel, angpos, acc, angacc, xyzsum written 168) come on top; its
         # reads of force, torque, pos, vel and angvel are gone
         bytes_per_particle += 272.0
-        kernel_name = "k_contacts_integrate (contact search + forces + integration)"
+        # the stage profile times this launch by itself; the timed steps run the
+        # same work inside k_step, which has no launch of its own to time
+        kernel_name = ("k_contacts_integrate (contact search + forces + integration), from the "
+                       "stage profile; the timed region runs its work in k_step")
         traffic = FUSED_TRAFFIC if precision == "mixed" else None
     contacts_bytes = n * bytes_per_particle
     achieved = contacts_bytes / (prof.contacts_ms * 1e-3) / 1e9
-    # launches of this library's kernels in the timed region: per DEM step
-    # k_resort (with the list rebuild), k_contacts, k_integrate (+2 for the
-    # shear-stress wall, +2 with bonds) on the per-stage path; one k_step, and a
-    # k_step_end per call, with contacts and integration in one launch (systems
-    # of one wave, as this one); one k_persistent per call on the persistent path
-    if info.step_path == 1:
-        timed_launches = args.steps
-    elif info.step_path == 2:
-        timed_launches = (INTERVAL + 1) * args.steps
-    else:
-        per_step = 3 + (2 if d.nw > 0 and d.wmode[0] == 3 else 0) + (2 if d.nb0 > 0 else 0)
-        timed_launches = per_step * INTERVAL * args.steps
     out = {
         "metric": "particle-steps/s",
         "value": value,
@@ -316,7 +322,7 @@ def run_gpu(args):
                    "l2": "flushed between timed steps (256 MB write)"},
         "e2e": {"value": e2e_value, "unit": "particle-steps/s",
                 "h2d_bytes_per_step": 3 * 32 * n, "d2h_bytes_per_step": 5 * 32 * n},
-        "gpu_launches": timed_launches,
+        "gpu_launches": timed_launches(info, d, args.steps),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak,
                      "traffic": traffic,
@@ -837,9 +843,6 @@ def run_distributed(args, rank, world):
     max_e2e = max_over_ranks(e2e_s, dev)
     comb = combine_replicas(max_ms, max_e2e, world, n, args.steps)
     if rank == 0:
-        per_step = 3 + (2 if d.nw > 0 and d.wmode[0] == 3 else 0)
-        if info.step_path == 2:
-            per_step = 3
         out = {
             "metric": "particle-steps/s", "value": comb["value"], "unit": "particle-steps/s",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
@@ -853,8 +856,7 @@ def run_distributed(args, rank, world):
                        "l2": "flushed between timed steps (256 MB write)"},
             "e2e": {"value": comb["e2e_value"], "unit": "particle-steps/s",
                     "h2d_bytes_per_step": 3 * 32 * n * world, "d2h_bytes_per_step": 3 * 32 * n * world},
-            "gpu_launches": (args.steps if info.step_path == 1
-                             else per_step * INTERVAL * args.steps) * world,
+            "gpu_launches": timed_launches(info, d, args.steps) * world,
             "clocks": clocks,
         }
         print(json.dumps(out), flush=True)

@@ -59,3 +59,16 @@ def test_step_path_names():
     assert name(0) == "per-stage"
     assert name(1) == "persistent"
     assert name(2) == "per-stage, contacts and integration in one launch"
+
+
+def test_launch_counts():
+    """gpu_launches of the benchmark line, of one job and of replicas: a call of
+    100 steps is 100 launches of the one-launch step and the one that ends it."""
+    import types
+    sys.path.insert(0, ROOT)
+    import bench
+    ns = types.SimpleNamespace
+    dry = ns(nw=1, wmode=[1], nb0=0)
+    count = lambda p, d: bench.timed_launches(ns(step_path=p), d, 20)  # noqa: E731
+    assert [count(p, dry) for p in (0, 1, 2)] == [6000, 20, 2020]
+    assert count(0, ns(nw=1, wmode=[3], nb0=0)) == count(0, ns(nw=0, wmode=[], nb0=5)) == 10000
