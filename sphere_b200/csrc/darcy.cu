@@ -1246,9 +1246,12 @@ int Engine::darcy_init()
     unsigned need = cells_blocks(D);
     if ((unsigned)jacobi_grid > need) jacobi_grid = (int)need;
     if ((unsigned)jacobi_grid > kJacobiMaxBlocks) jacobi_grid = (int)kJacobiMaxBlocks;
-    // k_jacobi_flow where its boundaries and registers allow: 40 x 40 x 80
-    // cells, 17,600 of them changing, 2.0 us per iteration against 6.7 of
-    // k_jacobi, whose blocks hand over through flags and fences
+    // k_jacobi_flow where its boundaries allow and any number of changing cells
+    // fits its registers: 40 x 40 x 80 cells, 17,600 of them changing, 2.0 us per
+    // iteration against 6.7 of k_jacobi, whose blocks hand over through flags and
+    // fences.  How many change is only known on the device, solve by solve (walls
+    // move, pressures are set), so the grid's size decides: a larger grid with as
+    // few changing cells would fit too
     auto closed = [](int b) { return b == 0 || b == 1; };
     const size_t ncell = nx * ny * nz;
     if (((D.bc_xn == 2 && D.bc_xp == 2) || (closed(D.bc_xn) && closed(D.bc_xp))) &&

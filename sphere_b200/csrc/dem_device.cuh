@@ -318,17 +318,17 @@ __device__ __forceinline__ void grid_pos(const DevParams &P, double4 x, int &gx,
 
 // ---------------------------------------------------------------------
 // contact search + forces: topology (contactsearch.cuh:329-371) and
-// interact (contactsearch.cuh:385-726) for one particle per thread.
+// interact (contactsearch.cuh:385-726), by warps (contact_warp below).
 //
 // Candidates come from a neighbour list built in the reference's visiting
 // order (27 cells z, y, x; sorted order inside a cell) holding every pair
 // closer than r_a + r_b + skin.  The list is rebuilt whenever the sort
 // changed or a particle moved more than 0.45 skin since the build, so a
-// pair missing from it cannot overlap: the overlap tests, and therefore the
-// slot insertions, happen in exactly the reference's sequence.  The slot
-// row is tracked with an occupancy bitmask so the slot policy and the force
-// loop visit occupied slots only; empty slots keep zero history, which is
-// what the reference rewrites into them every step.
+// pair missing from it cannot overlap: new contacts take their slots in exactly
+// the reference's sequence (one that finds its slot changes none).  An occupancy
+// bitmask per row (DevState::occ) lets the slot policy and the forces visit
+// occupied slots only; empty slots keep zero history, which is what the
+// reference rewrites into them every step.
 // ---------------------------------------------------------------------
 constexpr uint32_t NL_OVERFLOW = 0xffffffffu;
 
@@ -545,9 +545,9 @@ __device__ __forceinline__ bool touches(const DevParams &P, const double4 &xa, c
 //      the row;
 //   4. the owner adds its contacts' results in slot order, the reference's
 //      summation order, so every sum is formed as before, bit for bit.
-// Measured on the shear box (100,000 particles, B200, launch time): one
-// particle per thread 43 us mixed and 58 us faithful FP64; this 36 and 45 (400 spheres, 8 contacts each: 49 and
-// 14 us, and 54 and 18 us for the whole step).
+// Measured (B200, launch time of k_contacts, one particle per thread / this): the
+// shear box of 100,000 particles 43 / 39 us mixed and 58 / 45 us faithful FP64, 400
+// spheres with 8 contacts each 49 / 14 us.
 // PREC 0: faithful FP64, 1: FP64, 2: mixed (FP64 overlap, FP32 contact law,
 // FP64 accumulation).
 // before_walls() runs in all lanes once the contacts are done and before the
@@ -1493,9 +1493,14 @@ __device__ __forceinline__ bool wait_equal(const unsigned *p, unsigned want, Dev
 //
 // The wall forces per particle have two buffers, like x, vel and angvel.
 // Block 0 owns no particles; blocks 1.. take 4 pw each.
-// Measured (us per step, B200, three launches / this): 400 spheres 18.0 / 14.1,
-// 10,000 without contacts 16.1 / 13.9, 20,011 viscous 33.0 / 27.9, 100,000 in
-// shear 56.7 / 53.1 mixed and 72.1 / 63.1 faithful FP64.
+// Measured (us per step, B200, three launches / this): 400 spheres 18.0 / 14.3,
+// 10,000 without contacts 16.1 / 12.9, 20,011 viscous 33.0 / 28.0, 100,000 in
+// shear 56.7 / 50.2 mixed and 72.1 / 63.0 faithful FP64.
+//
+// Every form of the work is in this one kernel (re-sort, list build, both forms of
+// the integration), so at 80 registers it spills more than the kernels it
+// replaces: bytes of spill stores / loads 1048 / 1388 faithful (k_contacts_integrate
+// 944 / 1308, k_contacts alone 300 / 332) and 544 / 532 mixed (532 / 488, 260 / 216).
 template <int PREC, int MODEL>
 __global__ void __launch_bounds__(SPHB_CONTACT_B, SPHB_CONTACT_MINB)
 k_step(DevParams P, DevState S, PermScratch W, unsigned pw, int view, int pending)

@@ -2,7 +2,8 @@
 //
 // Compiled with -fmad=false: every expression keeps the reference's
 // operation order and rounding (the reference is built with --fmad=false,
-// src/CMakeLists.txt:25).  One thread per particle in sorted order.
+// src/CMakeLists.txt:25).  Particles in sorted order: the contact kernels share
+// them among the lanes of a warp (contact_warp), the others take one per thread.
 #include "dem_device.cuh"
 #include "contacts_staged.cuh"
 #include "contact_launch.cuh"
