@@ -23,7 +23,9 @@ extern "C" {
 
 typedef struct sph_engine sph_engine;
 
-/* Status codes. */
+/* Status codes.  After an error of a step (OUTSIDE, CAPACITY, TIMEOUT) a handle is
+ * good for reading and closing: on the step paths that integrate within the contact
+ * launch, particles may stand on either side of the step that failed. */
 enum {
     SPH_OK = 0,
     SPH_WARN_NOCONV = 1,        /* Darcy solve hit maxiter (the reference continues) */
