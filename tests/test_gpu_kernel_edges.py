@@ -36,8 +36,8 @@ def pressed(n, seed=61, model=2):
 
 # a B200 holds 148 x 24 = 3552 warps of these kernels: one particle per warp up
 # to 3552, two up to 7104, ... 16 up to 56832, then 32
-@pytest.mark.parametrize("n,model", [(1, 2), (31, 1), (33, 2), (3552, 2), (3553, 1), (7105, 2), (14209, 2),
-                                     (28417, 1), (56833, 2)])
+@pytest.mark.parametrize("n,model", [(1, 2), (31, 1), (33, 2), (3552, 2), (3553, 1), (7104, 1), (7105, 2),
+                                     (14208, 2), (14209, 2), (28416, 2), (28417, 1), (56832, 1), (56833, 2)])
 def test_particles_per_warp(tmp_path, n, model):
     from sphere_b200.engine import Engine
     d = pressed(n, model=model)
@@ -70,6 +70,24 @@ def test_render_tiles(n, w, h, scale):
             ref = R.render(x, vel, d.L, w, h, method=method, val=val, max_val=max_val)
             assert (ref[:, :, :3] != 255).any() or w < 16 or n == 1
             assert numpy.array_equal(img[:, :, :3], ref[:, :, :3]), (n, w, h, method)
+
+
+# the one-launch step leaves one of its 888 blocks to the walls: 3548 warps for the
+# particles; beyond 32 in each it takes three launches
+@pytest.mark.parametrize("n,model", [(3548, 2), (3549, 1), (7096, 2), (7097, 2), (14192, 1), (14193, 2),
+                                     (28384, 2), (28385, 1), (56768, 2), (56769, 2), (113536, 1), (113537, 2)])
+def test_particles_per_warp_of_one_launch_steps(tmp_path, n, model):
+    from sphere_b200.engine import Engine
+    d = pressed(n, model=model)
+    path = str(tmp_path / "edge.bin")
+    binfile.write_bin(d, path)
+    orc = O.Oracle(path)
+    with Engine(path, step_kernel="stages_fused") as e:
+        for steps in (1, 4):
+            assert orc.step(steps) == 0, orc.error()
+            assert e.step(steps) == 0
+            bad = compare(e, orc)
+            assert not bad, (n, bad)
 
 
 # a tile stages spheres 256 at a time and traces them when more than 256 are
