@@ -279,6 +279,9 @@ __global__ void __launch_bounds__(NT, MINB) k_persistent(BatchArgs A)
                 pc->flag_resort[(iter + 1) & 1] = 0;
                 pc->flag_nl[(iter + 1) & 1] = 0;
             }
+            // this step's errors are all raised, and no block has begun the next:
+            // every block reads the same and leaves the loop at the same step
+            if (t == 0) h.err = *(volatile int *)&S.ctl->err;
             if (P.nw > 0)
                 for (unsigned j = rank; j < box.nblk; j += gsz) {
                     double sj = chunk_tree_sum(S.walls_force_pp, P.np, j, cache);
@@ -290,7 +293,6 @@ __global__ void __launch_bounds__(NT, MINB) k_persistent(BatchArgs A)
             if (t == 0) {
                 DevCtl *ctl = S.ctl;
                 walls_integrate(P, S, wforce, iter, h.t_current);   // this block's copies
-                const int err = *(volatile int *)&ctl->err;
                 const int nres = *(volatile int *)fr, nnl = *(volatile int *)fn;
                 const double t_next = h.t_current + P.dt;
                 const int vs_next = next_velocity_state(h.velocity_state, h.t_current);
@@ -310,13 +312,12 @@ __global__ void __launch_bounds__(NT, MINB) k_persistent(BatchArgs A)
                     if (resorted) ctl->resorts += 1;
                     if (nl) ctl->nl_builds += 1;
                     pc->view = v ^ 1;
-                    if (err) atomicOr(A.any_err, 1);
+                    if (h.err) atomicOr(A.any_err, 1);
                     __threadfence();
                 }
                 h.iter = iter + 1;
                 h.t_current = t_next;
                 h.velocity_state = vs_next;
-                h.err = err;
                 h.resort = nres;
                 h.nl = nnl;
                 h.view = v ^ 1;

@@ -66,6 +66,14 @@ def test_overflow_leaves_the_steps_before_it_whole(shape):
             e.close()
         assert 4 < after[0][0] < 20
         assert after[0] == after[1]
+        # every block of the persistent kernel leaves at the same step
+        e = Engine(d, capacity=1, step_kernel="persistent")
+        assert e.step(3) == 0
+        with pytest.raises(EngineError) as exc:
+            e.step(20)
+        assert exc.value.status == -6
+        assert int(e.get("iter")[0]) == after[0][0] + 1     # the failing step counts
+        e.close()
 
 
 def test_particle_leaving_the_grid_is_reported():
